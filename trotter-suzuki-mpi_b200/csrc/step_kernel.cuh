@@ -499,71 +499,97 @@ __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 // Phase factors of the GPE / LHY term for small arguments.  The nonlinear
 // phase g*dt*|psi|^2 is far below 1/32 in practice, where truncated Maclaurin
 // series of cos, sin and exp (Horner's rule) leave a remainder well under half
-// an ulp; larger arguments take the CUDA math library.  Two tiers, chosen for
-// the whole warp:
+// an ulp; larger arguments take the CUDA math library.  Two tiers:
 //   |th| < 2^-8: double cos / sin to the t^3 terms (t = th^2), exp to x^6
 //                (remainders below 3e-21; Estrin's scheme, a shorter
 //                dependency chain than Horner's); float cos / sin to t^2,
 //                exp to x^4 (below 1e-14);
 //   |th| < 1/32: cos / sin to t^5, exp to x^8 (remainders below 1e-19).
-// Returns sin(th) and cos(th) (cos(th) - 1 in delta form).  The comparisons
-// are exact in either precision.
+// The warp takes the shortest that serves all its cells, or (CELL, sin and
+// cos) each cell its own: a warp whose cells are all in the first tier, the
+// usual case, evaluates that one only, another the second, and the cells in
+// the first tier or past the second replace its result.  With two branches
+// instead of three for the whole warp more of the row body is scheduled
+// across them: the 2048^2 double real-time step took 38.7 us against
+// 43.9-48.0 (phases of the second tier 46.6 / 49.7, of the library 65.2 /
+// 63.6).  Float gains nothing by it (25.5 / 25.9; library 47.7 / 43.7) and
+// nor does the double rotating frame (2048^2 74.7 / 73.6), which keep the
+// warp's choice.  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
+// The comparisons are exact in either precision.
 __device__ __forceinline__ bool phase_tiny(double th) { return fabs(th) < 0.00390625; }
 __device__ __forceinline__ bool phase_tiny(float th) { return fabsf(th) < 0.00390625f; }
 __device__ __forceinline__ bool phase_small(double th) { return fabs(th) < 0.03125; }
 __device__ __forceinline__ bool phase_small(float th) { return fabsf(th) < 0.03125f; }
 
-// TIERS = false: the 1/32 tier and the library only (less code, for the
-// kernels whose row body is long enough for instruction fetch to limit them).
-template <typename T, bool TIERS = true>
-__device__ __forceinline__ void phase_sincos(T th, T *s, T *c) {
-    constexpr bool F = std::is_same<T, float>::value;
-    // warp-uniform choice: the shorter series if every lane allows it, the
-    // library path only if some lane needs it
-    if (TIERS && !__any_sync(0xffffffffu, !phase_tiny(th))) {
-        const T t = th * th;
-        if (F) {
-            const T pc = fma_t(T(4.1666666666666664e-02), t, T(-0.5));               // 1/4!, -1/2!
-            const T ps = fma_t(T(8.3333333333333332e-03), t, T(-1.6666666666666666e-01));  // 1/5!, -1/3!
-            *c = DeltaForm<T>::value ? mul_t(pc, t) : fma_t(pc, t, T(1));
-            *s = fma_t(mul_t(ps, t), th, th);
-        } else {
-            // Estrin's scheme (two levels instead of Horner's three):
-            // cos = (1 - t/2!) + t^2 (1/4! - t/6!),
-            // sin = th + (th t) ((-1/3! + t/5!) - t^2/7!)
-            const T t2 = mul_t(t, t);
-            const T c0 = fma_t(t, T(-0.5), T(1));
-            const T c1 = fma_t(t, T(-1.3888888888888889e-03), T(4.1666666666666664e-02));
-            const T s0 = fma_t(t, T(8.3333333333333332e-03), T(-1.6666666666666666e-01));
-            const T ps = fma_t(t2, T(-1.9841269841269841e-04), s0);
-            *c = fma_t(c1, t2, c0);
-            *s = fma_t(mul_t(th, t), ps, th);
-        }
-    } else if (!__any_sync(0xffffffffu, !phase_small(th))) {
-        const T t = th * th;
-        T pc = T(-2.7557319223985893e-07);            // -1/10!
-        pc = fma_t(pc, t, T(2.4801587301587302e-05));  //  1/8!
-        pc = fma_t(pc, t, T(-1.3888888888888889e-03)); // -1/6!
-        pc = fma_t(pc, t, T(4.1666666666666664e-02));  //  1/4!
-        pc = fma_t(pc, t, T(-0.5));                    // -1/2!
-        T ps = T(-2.5052108385441720e-08);             // -1/11!
-        ps = fma_t(ps, t, T(2.7557319223985888e-06));  //  1/9!
-        ps = fma_t(ps, t, T(-1.9841269841269841e-04)); // -1/7!
-        ps = fma_t(ps, t, T(8.3333333333333332e-03));  //  1/5!
-        ps = fma_t(ps, t, T(-1.6666666666666666e-01)); // -1/3!
+template <typename T>
+__device__ __forceinline__ void sincos_tiny(T th, T *s, T *c) {
+    const T t = th * th;
+    if constexpr (std::is_same<T, float>::value) {
+        const T pc = fma_t(T(4.1666666666666664e-02), t, T(-0.5));               // 1/4!, -1/2!
+        const T ps = fma_t(T(8.3333333333333332e-03), t, T(-1.6666666666666666e-01));  // 1/5!, -1/3!
         *c = DeltaForm<T>::value ? mul_t(pc, t) : fma_t(pc, t, T(1));
         *s = fma_t(mul_t(ps, t), th, th);
     } else {
-        sincos_t(th, s, c);
-        if (DeltaForm<T>::value) {
-            // cos(th) - 1 = -2 sin^2(th / 2), without cancellation
-            const T h = sin_t(T(0.5) * th);
-            *c = T(-2) * h * h;
-        }
+        // Estrin's scheme (two levels instead of Horner's three):
+        // cos = (1 - t/2!) + t^2 (1/4! - t/6!),
+        // sin = th + (th t) ((-1/3! + t/5!) - t^2/7!)
+        const T t2 = mul_t(t, t);
+        const T c0 = fma_t(t, T(-0.5), T(1));
+        const T c1 = fma_t(t, T(-1.3888888888888889e-03), T(4.1666666666666664e-02));
+        const T s0 = fma_t(t, T(8.3333333333333332e-03), T(-1.6666666666666666e-01));
+        const T ps = fma_t(t2, T(-1.9841269841269841e-04), s0);
+        *c = fma_t(c1, t2, c0);
+        *s = fma_t(mul_t(th, t), ps, th);
     }
 }
 
-// exp(-th) for the imaginary-time nonlinear factor (same tiers).
+template <typename T>
+__device__ __forceinline__ void sincos_small(T th, T *s, T *c) {
+    const T t = th * th;
+    T pc = T(-2.7557319223985893e-07);            // -1/10!
+    pc = fma_t(pc, t, T(2.4801587301587302e-05));  //  1/8!
+    pc = fma_t(pc, t, T(-1.3888888888888889e-03)); // -1/6!
+    pc = fma_t(pc, t, T(4.1666666666666664e-02));  //  1/4!
+    pc = fma_t(pc, t, T(-0.5));                    // -1/2!
+    T ps = T(-2.5052108385441720e-08);             // -1/11!
+    ps = fma_t(ps, t, T(2.7557319223985888e-06));  //  1/9!
+    ps = fma_t(ps, t, T(-1.9841269841269841e-04)); // -1/7!
+    ps = fma_t(ps, t, T(8.3333333333333332e-03));  //  1/5!
+    ps = fma_t(ps, t, T(-1.6666666666666666e-01)); // -1/3!
+    *c = DeltaForm<T>::value ? mul_t(pc, t) : fma_t(pc, t, T(1));
+    *s = fma_t(mul_t(ps, t), th, th);
+}
+
+template <typename T>
+__device__ __forceinline__ void sincos_large(T th, T *s, T *c) {
+    sincos_t(th, s, c);
+    if (DeltaForm<T>::value) {
+        // cos(th) - 1 = -2 sin^2(th / 2), without cancellation
+        const T h = sin_t(T(0.5) * th);
+        *c = T(-2) * h * h;
+    }
+}
+
+// TIERS = false: the 1/32 tier and the library only (less code, for the
+// kernels whose row body is long enough for instruction fetch to limit them).
+template <typename T, bool TIERS = true, bool CELL = std::is_same<T, double>::value>
+__device__ __forceinline__ void phase_sincos(T th, T *s, T *c) {
+    if (TIERS && !__any_sync(0xffffffffu, !phase_tiny(th))) {
+        sincos_tiny(th, s, c);
+    } else if (CELL) {
+        sincos_small(th, s, c);
+        if (TIERS && phase_tiny(th)) sincos_tiny(th, s, c);
+        else if (!phase_small(th)) sincos_large(th, s, c);
+    } else if (!__any_sync(0xffffffffu, !phase_small(th))) {
+        sincos_small(th, s, c);
+    } else {
+        sincos_large(th, s, c);
+    }
+}
+
+// exp(-th) for the imaginary-time nonlinear factor: the same tiers by the
+// warp's choice (by the cell's, 2048^2 double with large phases took 56.9 us
+// against 49.3).
 template <typename T, bool TIERS = true>
 __device__ __forceinline__ T phase_expneg(T th) {
     constexpr bool F = std::is_same<T, float>::value;
@@ -705,8 +731,8 @@ __device__ __forceinline__ Cx<T> rabi_cell(Cx<T> self, Cx<T> other, T cc, T sr, 
 // PB (two components): the phase adds g_ab dt |psi_b|^2, psi_b the other
 // species' cell at the start of this step (`ub`, already scaled)
 // (src/cpucartesian.cpp:73-92,113-126).
-template <bool IMAG, bool PHASE, bool LHY, bool PB, int C, bool TIERS = true, typename T,
-          typename TabT>
+template <bool IMAG, bool PHASE, bool LHY, bool PB, int C, bool TIERS = true, bool ROT = false,
+          typename T, typename TabT>
 __device__ __forceinline__ void potential_row(Cx<T> (&w)[C], const TabT *tab, T ca, T caa,
                                               const Cx<T> (*ub)[C] = nullptr, T cab = T(0)) {
     if constexpr (IMAG && PHASE && std::is_same<T, float>::value && C % 2 == 0) {
@@ -760,7 +786,7 @@ __device__ __forceinline__ void potential_row(Cx<T> (&w)[C], const TabT *tab, T 
                 T th = mul_t(ca, n2);
                 if (LHY) th = fma_t(caa, mul_t(n2, sqrt_t(n2)), th);
                 if (PB) th = th + thb;
-                phase_sincos<T, TIERS>(th, &s, &c);
+                phase_sincos<T, TIERS, std::is_same<T, double>::value && !ROT>(th, &s, &c);
             }
             // the table holds (cos, sin) of -dt V; in delta form (cos - 1, sin):
             // v (cos + i sin), the kinetic pair's form with the cell as its own
@@ -992,7 +1018,7 @@ __device__ __forceinline__ void walk_row(Walk<V> &w, const StepArgs<typename V::
             }
             potential_row<IMAG, PHASE, false, true, C, false>(WS(2), tp, w.ca, w.caa, &ub, w.cab);
         } else {
-            potential_row<IMAG, PHASE, V::LHY, false, C>(WS(2), tp, w.ca, w.caa);
+            potential_row<IMAG, PHASE, V::LHY, false, C, true, ROT>(WS(2), tp, w.ca, w.caa);
         }
         if constexpr (ROT) {
             const Cx<T> ab = reinterpret_cast<const Cx<T> *>(a.row_ab)[u];

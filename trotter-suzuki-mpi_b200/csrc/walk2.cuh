@@ -348,7 +348,7 @@ __device__ __forceinline__ void w2_stages(Walk2<V, R> &w, int t) {
             load_tab_cells<TabT, C>(w.ring + q * S::SLOT + pos * S::ROWB + V::PSI_BYTES +
                                         C * (int)sizeof(TabT) * w.lane,
                                     tv);
-            potential_row<IMAG, PHASE, V::LHY, false, C>(W2S(2), tv, w.ca, w.caa);
+            potential_row<IMAG, PHASE, V::LHY, false, C, true, true>(W2S(2), tv, w.ca, w.caa);
             const Cx<T> ab = Walk2<V, R>::AB_AHEAD ? w.rab[(K + 2) % 4] : w2_row_ab(w, c - 2);
             rrow<IMAG, C, 0, true>(W2S(2), ab.re, ab.im, w.m);
             rrow<IMAG, C, 1, true>(W2S(2), ab.re, ab.im, w.m);
