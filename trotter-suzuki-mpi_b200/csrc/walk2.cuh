@@ -137,6 +137,7 @@ struct Walk2 {
     uint32_t psi_off, psi_bytes, tab_off, tab_bytes;
     int H;
     unsigned char *ring;
+    bool fresh;  // no copy has landed in the ring since it was zeroed
     Cx<T> *vco;
     uint64_t *bars;
     Cx<T> *orow;  // row oy0 - 8 of the output at this lane's first column (moved per row)
@@ -687,24 +688,25 @@ __device__ __forceinline__ void w2_task(Walk2<V, R> &w, const StepArgs<typename 
     }
     w.orow = reinterpret_cast<Cx<T> *>(a.psi_out) + (ptrdiff_t)(oy0 - S::SO) * a.P + xl;
     __syncwarp();  // the previous task's reads of the ring are done
-    if (c0 < 0 || c0 + S::SW > a.P) {
-        // cells of the strip outside the tile read as 0 (copies do not cover them)
-        uint32_t *ring32 = reinterpret_cast<uint32_t *>(w.ring);
-        for (int i = lane; i < S::D * S::SLOT / 4; i += 32) {
-            const uint32_t off = (uint32_t)(i * 4) % (uint32_t)S::ROWB;
-            bool copied;
-            if (off < (uint32_t)V::PSI_BYTES) {
-                copied = off >= w.psi_off && off < w.psi_off + w.psi_bytes;
-            } else if (off < (uint32_t)S::PB_OFF) {
-                const uint32_t tt = off - (uint32_t)V::PSI_BYTES;
-                copied = tt >= w.tab_off && tt < w.tab_off + w.tab_bytes;
-            } else {
-                const uint32_t tt = off - (uint32_t)S::PB_OFF;
-                copied = tt >= w.psi_off && tt < w.psi_off + w.psi_bytes;
-            }
-            if (!copied) ring32[i] = 0u;
+    if (!w.fresh && (c0 < 0 || c0 + S::SW > a.P)) {
+        // cells of the strip outside the tile read as 0: the copies do not
+        // cover them, an earlier task's may have (a fresh ring is zero: a
+        // warp's first task, the edge strips' with one task per warp, starts
+        // its copies some 2 us earlier than with a pass over the ring).  The
+        // copied regions are multiples of 16 bytes.
+        auto clear = [&](unsigned char *p, uint32_t bytes, uint32_t off, uint32_t n) {
+            for (uint32_t o = 16u * (uint32_t)lane; o < bytes; o += 512u)
+                if (o < off || o >= off + n)
+                    *reinterpret_cast<uint4 *>(p + o) = make_uint4(0u, 0u, 0u, 0u);
+        };
+        for (int r = 0; r < S::NW; ++r) {
+            unsigned char *row = w.ring + r * S::ROWB;
+            clear(row, V::PSI_BYTES, w.psi_off, w.psi_bytes);
+            clear(row + V::PSI_BYTES, V::TAB_BYTES, w.tab_off, w.tab_bytes);
+            if constexpr (V::PB) clear(row + S::PB_OFF, V::PSI_BYTES, w.psi_off, w.psi_bytes);
         }
     }
+    w.fresh = false;
     __syncwarp();
     if (lane == 0) {
         // fresh barriers: every slot starts at phase 0 for this task
@@ -863,6 +865,7 @@ __device__ __forceinline__ void w2_warp_setup(Walk2<V, R> &w, unsigned char *sme
     w.lane = lane;
     w.nacc = 0.0;
     w.failed = false;
+    w.fresh = true;
     w.ring = smem + (size_t)warp * S::D * S::SLOT;
     w.vco = reinterpret_cast<Cx<T> *>(smem + (size_t)warps * S::D * S::SLOT) + (size_t)warp * vl;
     w.bars = reinterpret_cast<uint64_t *>(smem + (size_t)warps * S::D * S::SLOT +
