@@ -272,6 +272,12 @@ __global__ void copy_tile_kernel(Cx<T> *dst, size_t dpitch, const Cx<T> *src, si
 template <typename T>
 __global__ void halo_kernel(Cx<T> *psi, int W, int H, int P, int hx, int hy, int px, int py,
                             int xr0, int xr1) {
+    // launched with a programmatic dependency on the step: its blocks are in
+    // place when the step ends (periodic 2048^2 float real time 29.4 -> 28.0
+    // us per step, 1300^2 double 23.8 -> 23.1); not in a rotating frame, whose
+    // float step it slowed (4096^2 152.9 -> 153.9)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     tsb::halo_cells(psi, W, H, P, hx, hy, px, py, xr0, xr1, blockIdx.x * blockDim.x + threadIdx.x,
                     gridDim.x * blockDim.x);
 }
@@ -720,10 +726,18 @@ int launch_halo_t(ts_b200_kernel *k, cudaStream_t stream = nullptr, int xr0 = 0,
     if (n <= 0) return TS_B200_OK;
     const int threads = 256;
     const int nb = std::min(div_up(n, threads), 4096);
-    halo_kernel<T><<<nb, threads, 0, stream>>>(reinterpret_cast<Cx<T> *>(k->psi[k->cur]), k->W,
-                                                  k->H, k->P, hx, hy, k->d.periodic_x,
-                                                  k->d.periodic_y, xr0, xr1);
-    cudaError_t e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nb);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = k->rot ? 0 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, halo_kernel<T>,
+                                       reinterpret_cast<Cx<T> *>(k->psi[k->cur]), k->W, k->H, k->P,
+                                       hx, hy, (int)k->d.periodic_x, (int)k->d.periodic_y, xr0, xr1);
     if (e != cudaSuccess) return cuda_fail(k, e, "halo kernel launch");
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TS_B200_OK;
