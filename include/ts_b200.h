@@ -313,7 +313,9 @@ int ts_b200_synchronize(ts_b200_kernel *k);
 
 /* Geometry of the fused step launch chosen for this tile (for reporting):
  * cells per lane, rows per segment, warps per block, ring depth, tasks, and
- * the row walk (0 checked; 1 or 2: look-ahead, rows per iteration). */
+ * the row walk (0 checked; 1 or 2: look-ahead, rows per iteration).  walk 3:
+ * register patches; then cells_per_lane is the side of a thread's patch,
+ * strips x segments the regions, segment_rows the rows that one writes. */
 typedef struct {
     int32_t cells_per_lane, segment_rows, warps_per_block, ring_depth;
     int32_t strips, segments, blocks, threads;
@@ -329,7 +331,10 @@ int ts_b200_set_launch(ts_b200_kernel *k, int cells_per_lane, int segment_rows, 
                        int ring_depth);
 
 /* Row walk of the fused step (no counterpart in the reference; every walk
- * performs the same operations per cell): 2 (default) the look-ahead walk of
+ * performs the same operations per cell).  By default small and middle-sized
+ * tiles are stepped by register patches (a block holds a region of the tile
+ * in registers; launch info reports walk 3) and larger ones by walk 2; a call
+ * of this or of ts_b200_set_launch chooses a row walk: 2 the look-ahead walk of
  * every variant, with even segments, a ring of 6 rows (8 in a rotating
  * frame), 4 or 8 warps per block (4 in a rotating frame) and two rows per
  * iteration (one mbarrier per row pair; with 4 cells per lane one row,
@@ -339,8 +344,9 @@ int ts_b200_set_launch(ts_b200_kernel *k, int cells_per_lane, int segment_rows, 
  * the checked walk). */
 int ts_b200_set_walk(ts_b200_kernel *k, int walk);
 
-/* The look-ahead walk launches each fused step with a programmatic
- * dependency on the previous kernel of the stream (on = 1, the default): the
+/* The look-ahead walk and the register patches launch each fused step with a
+ * programmatic dependency on the previous kernel of the stream (on = 1; by
+ * default where it was measured faster): the
  * step's blocks are scheduled as the previous step's blocks retire and set up
  * their shared memory, then wait for the previous kernel to complete before
  * they read the tile.  on = 0 launches each step after the previous kernel

@@ -1,0 +1,203 @@
+"""The register-patch step against the checked walk and the oracle.
+
+The patches perform the same operations per cell as the row walks (the same
+pair forms, potential row and fused multiply-adds), so in real time a tile
+stepped by them carries the checked walk's bits; in imaginary time the squared
+norm is summed over another grid of blocks, so the renormalisation factor may
+differ in its last bits (1e-13).  The oracle bar is the parity bar, 1e-10.
+Sizes lie at the edges of the regions (24 or 56 written cells, 16 or 48 with 8
+halo columns) and on either side of the limits between patch sizes.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import desc_from_params, seeded_case
+
+pytestmark = pytest.mark.gpu
+
+# name, N, Ny, periodic, g, lhy, omega, imag, precision, patch side (cells 10/N
+# wide; in float imaginary time 0.16, where dt / (4 dx^2) = 0.01: at 1.8, as 853
+# columns over 10 would have it, eight sweeps of cosh(1.8) lose all of float)
+CASES = [
+    ("one_cell", 1, 1, (False, False), 1.0, 0.0, 0.0, False, 0, 2),
+    ("one_row", 50, 1, (False, False), 1.0, 0.0, 0.0, False, 0, 2),
+    ("one_column", 1, 50, (False, False), 0.0, 0.0, 0.0, True, 0, 2),
+    ("region", 24, 24, (False, False), 5.0, 0.3, 0.0, False, 0, 2),
+    ("region_plus_1", 25, 49, (False, False), 5.0, 0.0, 0.0, True, 0, 2),
+    ("rim_left", 27, 75, (False, False), 2.0, 0.0, 0.0, False, 0, 2),
+    ("interior", 130, 101, (False, False), 2.0, 0.0, 0.0, True, 0, 2),
+    ("interior_fp32", 131, 100, (False, False), 2.0, 0.1, 0.0, False, 1, 2),
+    ("linear_fp32", 77, 60, (False, False), 0.0, 0.0, 0.0, True, 1, 2),
+    ("wide_fp32", 850, 801, (False, False), 2.0, 0.0, 0.0, False, 1, 4),
+    ("wide_imag_fp32_coarse", 853, 802, (False, False), 2.0, 0.0, 0.0, True, 1, 4),
+    ("periodic", 64, 40, (True, True), 2.0, 0.0, 0.0, False, 0, 2),
+    ("periodic_odd", 63, 45, (True, True), 1.0, 0.0, 0.0, False, 0, 2),
+    ("periodic_odd_fp32", 63, 45, (True, True), 1.0, 0.0, 0.0, False, 1, 2),
+    ("periodic_x", 61, 30, (True, False), 1.0, 0.0, 0.0, True, 0, 2),
+    ("periodic_y", 30, 61, (False, True), 1.0, 0.0, 0.0, False, 0, 2),
+    ("halo_only", 4, 4, (True, True), 1.0, 0.0, 0.0, False, 0, 2),
+    ("rotating", 48, 33, (False, False), 3.0, 0.0, 0.6, False, 0, 2),
+    ("rotating_periodic", 70, 61, (True, True), 3.0, 0.0, 0.6, True, 0, 2),
+    ("rotating_wide", 345, 341, (True, True), 3.0, 0.2, 0.6, False, 0, 4),
+    ("rotating_wide_closed", 351, 350, (False, False), 0.0, 0.0, 0.6, False, 0, 4),
+    ("rotating_wide_fp32", 345, 341, (True, True), 3.0, 0.0, 0.6, False, 1, 4),
+]
+
+
+def _close(got, old, imag):
+    if imag:
+        assert np.abs(got - old).max() <= 1e-13 * np.abs(old).max()
+    else:
+        assert np.array_equal(got, old)
+
+
+@pytest.mark.parametrize("case", CASES, ids=[c[0] for c in CASES])
+def test_patches_match_checked_walk_and_oracle(case):
+    """40 steps in two evolve calls: plain launches and a replayed graph."""
+    from trottersuzuki_b200 import Kernel
+    _, N, Ny, per, g, lhy, omega, imag, prec, side = case
+    length = 0.16 * N if imag and prec else (10.0 if N > 4 else 1.0)
+    lat, psi0, V = seeded_case(N, length, Ny, per, omega)
+    n0 = O.expectations(lat, psi0)["norm2"] if imag else 0.0
+    p = lat.params(1e-3, imag, 1.0, g, lhy, omega, norm0=n0)
+    tr, ti = O.exp_table(V, 1e-3, imag)
+    out = {}
+    for walk in (None, 0):
+        with Kernel(desc_from_params(p, prec)) as k:
+            if walk is not None:
+                k.set_walk(walk)
+            else:
+                shape = k.launch_shape()
+                assert shape["walk"] == 3 and shape["cells_per_lane"] == side
+            k.set_state(psi0)
+            k.set_exp_potential(tr, ti)
+            k.evolve(3)
+            k.evolve(37)
+            out[walk] = k.get_state()
+    if prec == 0:
+        _close(out[None], out[0], imag)
+        ref = O.evolve(p, O.evolve(p, psi0, tr, ti, 3), tr, ti, 37)
+        assert np.abs(out[None] - ref).max() <= 1e-10
+    elif not imag:
+        assert np.array_equal(out[None], out[0])
+    else:
+        # a last-bit difference of the factor, rounded to float per step
+        assert np.abs(out[None] - out[0]).max() <= 40 * 2.0 ** -23 * np.abs(out[0]).max()
+
+
+@pytest.mark.parametrize("imag", [False, True], ids=["real", "imag"])
+@pytest.mark.parametrize("N,Ny,py,side", [(40, 37, False, 2), (47, 49, True, 2),
+                                          (270, 261, False, 2), (330, 310, False, 4)])
+def test_patches_on_cylinders(N, Ny, py, side, imag):
+    from trottersuzuki_b200 import Kernel
+    lat = O.Lattice(N, 8.0, Ny, 10.0, False, py, cylindrical=True)
+    X, Y = lat.coordinates()
+    rng = np.random.default_rng(5)
+    psi0 = np.exp(-((X - 2.0) ** 2 + Y ** 2) / 3.0) * (1 + 0.05 * rng.uniform(-1, 1, lat.shape))
+    psi0 = psi0 * np.exp(0.3j * Y)
+    V = 0.5 * (X ** 2 + Y ** 2) + lat.azimuthal(1)
+    n0 = O.expectations(lat, psi0)["norm2"] if imag else 0.0
+    p = lat.params(1e-3, imag, 1.0, 25.0, 0.0, 0.0, norm0=n0, angular_momentum=1)
+    tr, ti = O.exp_table(V, 1e-3, imag)
+    ref = O.evolve(p, O.evolve(p, psi0, tr, ti, 6), tr, ti, 36)
+    out = {}
+    for walk in (None, 0):
+        with Kernel(desc_from_params(p)) as k:
+            if walk is not None:
+                k.set_walk(walk)
+            else:
+                shape = k.launch_shape()
+                assert shape["walk"] == 3 and shape["cells_per_lane"] == side
+            k.set_state(psi0)
+            k.set_exp_potential(tr, ti)
+            k.evolve(6)
+            k.evolve(36)
+            out[walk] = k.get_state()
+    assert np.abs(out[None] - ref).max() <= 1e-10 * np.abs(ref).max()
+    _close(out[None], out[0], imag)
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("N,per,omega", [(40, (False, False), (5.0, 2.0)),
+                                         (57, (True, True), (0.0, 0.0)),
+                                         (430, (False, False), (5.0, 2.0))])
+def test_patches_of_a_pair(N, per, omega, prec):
+    """Two species with and without a Rabi coupling: the checked walk's bits
+    (430: 324 regions of 2 x 2 patches, 64 of 4 x 4)."""
+    from trottersuzuki_b200 import Kernel, Pair
+    lat, a0, V = seeded_case(N, 10.0, None, per)
+    b0 = np.roll(a0, 3, axis=1)
+    tr, ti = O.exp_table(V, 1e-3, False)
+    out = {}
+    for walk in (None, 0):
+        pa, pb = lat.params(1e-3, False, 1.0, 3.0), lat.params(1e-3, False, 1.2, 2.0)
+        with Kernel(desc_from_params(pa, prec)) as a, Kernel(desc_from_params(pb, prec)) as b:
+            for k, psi in ((a, a0), (b, b0)):
+                if walk is not None:
+                    k.set_walk(walk)
+                k.set_state(psi)
+                k.set_exp_potential(tr, ti)
+            with Pair(a, b, 4.0, omega[0], omega[1], 1e-3) as pair:
+                assert a.launch_shape()["walk"] == (3 if walk is None else 0)
+                pair.rabi(0.5)
+                pair.evolve(7)
+                pair.evolve(4)
+            out[walk] = (a.get_state(), b.get_state())
+    assert np.array_equal(out[None][0], out[0][0])
+    assert np.array_equal(out[None][1], out[0][1])
+
+
+@pytest.mark.parametrize("W,H", [(24, 24), (26, 51), (130, 100)])
+@pytest.mark.parametrize("pad", [0, 2])
+def test_patches_with_potential_rows(W, H, pad):
+    """Steps that read the potential (rows of any even pitch): the bits of a
+    table per step on the checked walk."""
+    import torch
+    from trottersuzuki_b200 import Kernel
+    lat, psi0, V = seeded_case(W, 10.0, H)
+    p = lat.params(1e-3, False, 1.0, 3.0, 0.2)
+    tr, ti = O.exp_table(V, 1e-3, False)
+    stack = torch.zeros((5, H, W + pad), dtype=torch.float64, device="cuda")
+    for i in range(5):
+        stack[i, :, :W] = torch.tensor(V * (1 + 0.1 * i))
+    torch.cuda.synchronize()
+    out = {}
+    for walk in (None, 0):
+        with Kernel(desc_from_params(p)) as k:
+            if walk is not None:
+                k.set_walk(walk)
+            k.set_state(psi0)
+            k.set_exp_potential(tr, ti)
+            k.evolve_potentials(stack.data_ptr(), W + pad, stack.stride(0), 5, 1e-3)
+            k.evolve(2)
+            out[walk] = k.get_state()
+    assert np.array_equal(out[None], out[0])
+
+
+def test_asking_for_a_walk_or_overlap_after_steps_keeps_the_evolution():
+    """Switches of walk and launch mode between evolve calls that replay graphs."""
+    from trottersuzuki_b200 import Kernel
+    from trottersuzuki_b200._capi import lib
+    lat, psi0, V = seeded_case(100, 10.0, 90, (True, True))
+    p = lat.params(1e-3, False, 1.0, 2.0)
+    tr, ti = O.exp_table(V, 1e-3, False)
+    res = []
+    for switch in (False, True):
+        with Kernel(desc_from_params(p)) as k:
+            k.set_state(psi0)
+            k.set_exp_potential(tr, ti)
+            k.evolve(70)
+            if switch:
+                assert lib().ts_b200_set_overlap(k.handle, C.c_int(1)) == 0
+            k.evolve(70)
+            if switch:
+                k.set_walk(2)
+                assert k.launch_shape()["walk"] == 2
+            k.evolve(70)
+            k.step(True)
+            k.step(False)
+            res.append(k.get_state())
+    assert np.array_equal(res[0], res[1])

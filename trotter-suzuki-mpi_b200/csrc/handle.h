@@ -41,7 +41,13 @@ struct ts_b200_kernel {
     int C = 2, seg_h = 64, warps = 4, ring = 4;
     int resident_blocks = 0;  // blocks of the current launch shape resident on the GPU (0: unknown)
     bool auto_seg = true;     // pick the segment height from the resident grid
-    bool overlap = true;      // look-ahead walk: programmatic dependent launch of each step
+    bool overlap = true;      // programmatic dependent launch of each step of a row walk
+    bool overlap_set = false; // overlap was asked for (it then holds for the patch step too)
+    bool patch = true;        // the register-patch step (patch.cuh) where it covers the variant;
+                              // off once a row walk or its shape has been asked for
+    // inside ts_b200_evolve: exchanging steps leave the halo to the next step
+    // (wrap_steps), whose input's halo is then not refreshed (wrap_next)
+    bool wrap_steps = false, wrap_next = false;
     int walk2 = 2;            // rows per iteration of the look-ahead walk (walk2.cuh) where
                               // the variant has one; 0: the checked walk
     cudaGraphExec_t graph = nullptr;

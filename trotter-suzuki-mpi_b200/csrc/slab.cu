@@ -265,7 +265,8 @@ int plan(ts_b200_slabs *s) {
         TSS_OK(plan_tile(s, x));
         const ts_b200_kernel *k = x.k;
         sig.insert(sig.end(), {(long long)k->C, k->seg_h, k->warps, k->ring, k->walk2,
-                               k->resident_blocks, (long long)(k->d.norm0 * 1e6), x.split,
+                               k->resident_blocks, k->patch, k->overlap, k->overlap_set,
+                               (long long)(k->d.norm0 * 1e6), x.split,
                                (long long)(uintptr_t)k->psi[0], (long long)(uintptr_t)k->psi[1],
                                (long long)(uintptr_t)x.scratch});
         s->launches_per_step += (x.split ? 2 : 1) + (k->d.periodic_x ? 1 : 0);

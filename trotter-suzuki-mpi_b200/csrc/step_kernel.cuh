@@ -118,6 +118,11 @@ struct StepArgs {
     // variants that read V instead of the table (phase bit 16), dt
     size_t pot_pitch;
     double pot_dt;
+    // register-patch step: the input's periodic halo has not been refreshed
+    // (bit 1 x, bit 2 y): its cells, wrap_hx columns (of the rows whose source
+    // lies in [wrap_y0, wrap_y1)) and wrap_hy rows on either side, are read
+    // from the cells that the refresh copies into them
+    int wrap, wrap_hx, wrap_hy, wrap_y0, wrap_y1;
 };
 
 // Output rows [oy0, oy1) of segment `seg` of the launch.

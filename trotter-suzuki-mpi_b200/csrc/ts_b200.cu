@@ -21,6 +21,7 @@
 #include "handle.h"
 #include "halo.cuh"
 #include "step_launch.h"
+#include "patch_decl.h"
 #include "step2_decl.h"
 #include "ts_b200.h"
 
@@ -663,6 +664,14 @@ void auto_segments(ts_b200_kernel *k) {
     k->seg_h = std::min(kMaxAutoSegment, balanced_segments(k, std::min(4, bps), k->warps));
 }
 
+// Programmatic dependent launch of a row walk's steps: where it was asked for
+// (ts_b200_set_overlap, the autotuner), else as measured (choose_launch) and
+// for steps queued one by one, whose launch gaps it hides (pairs in double
+// real time: 1024^2 53.4 -> 48.3 us per step; potential rows 27.1 -> 24.9).
+bool walk_pdl(const ts_b200_kernel *k) {
+    return k->overlap_set ? k->overlap : (k->overlap || k->pair_mode || k->vpot);
+}
+
 // pad: the shared memory of a launch with programmatic dependent launch
 // (padded to the grid's share of blocks per SM); without it, the kernel's own
 // need (for the occupancy that chooses the shape).
@@ -691,7 +700,7 @@ void geometry(const ts_b200_kernel *k, int *strips, int *segs, int *blocks, size
                                                                 (k->phase & 3) == 3) +
                                     tsb::w2_vlen(eff_seg(k), k->rot) * 2 * (k->fp32 ? 4 : 8) +
                                     (walk_window(k) / walk_rows(k)) * 8);
-        if (k->overlap && pad) {
+        if (walk_pdl(k) && pad) {
             // with programmatic dependent launch the next step's blocks are
             // placed as soon as an SM has room: reserve enough shared memory
             // that no SM holds more blocks of this step and the next together
@@ -803,6 +812,90 @@ template void tsbh::fill_step_constants<float>(const ts_b200_kernel *, StepArgs<
 
 namespace {
 
+// Regions of the patch step with patches of n x n cells.
+int patch_regions(const ts_b200_kernel *k, int n, int *nx, int *ny) {
+    *nx = div_up(k->W, tsb::patch_out(n, (k->rot || k->cyl) ? 8 : 4));  // Variant::HX
+    *ny = div_up(k->H, tsb::patch_out(n, k->rot ? 6 : 4));              // Variant::HY
+    return (long)*nx * *ny > INT32_MAX ? INT32_MAX : *nx * *ny;
+}
+
+// Cells per side of a thread's patch in the register-patch step (patch.cuh),
+// 0 where a row walk steps the tile: on large tiles, and where a walk or its
+// shape has been asked for.  Patches of 2 x 2 cells have the shorter latency,
+// of 4 x 4 fewer recomputed cells, the walk the best throughput.  The limits
+// are the region counts up to which each was the fastest of the three on
+// square tiles (us per step, 2 x 2 / 4 x 4 / walk):
+//   double, 4 halo columns: 256^2 3.3 / 8.4 / 9.3, 512^2 6.2 / 8.7 / 10.9,
+//     1024^2 15.1 / 18.8 / 18.2, 1280^2 26.0 / 23.6 / 21.5; imaginary time
+//     1024^2 17.3 / 19.0 / 18.8; potential rows 1024^2 19.2 / 28.0 / 24.9
+//   one species of a pair: 768^2 18.0 / 21.0 / 19.4, 1024^2 26.7 / 34.5 / 24.1;
+//     float 1024^2 20.3 / 17.6 / 18.9
+//   rotating frame, double: 256^2 5.8 / 10.1 / 18.9, 512^2 13.3 / 10.6 / 20.7,
+//     1024^2 41.7 / 25.6 / 32.0, 1300^2 - / 40.3 / 41.6
+//   rotating frame, float: 256^2 6.6 / 9.4 / 26.3, 512^2 11.0 / 9.8 / 26.5,
+//     2048^2 96.1 / 47.6 / 59.9, 4096^2 388 / 171 / 152
+//   cylinder, double: 256^2 7.7 / 11.0 / 12.7, 512^2 13.3 / 12.2 / 14.3,
+//     768^2 21.0 / 15.8 / 17.1, 1024^2 32.1 / 26.2 / 24.6
+//   cylinder, float: 512^2 9.8 / 9.1 / 11.4, 1536^2 39.6 / 23.2 / 24.1
+//   float, 4 halo columns: 512^2 6.5 / 8.1 / 9.2, 768^2 9.1 / 10.1 / 10.5,
+//     1024^2 13.3 / 11.7 / 13.8, 1536^2 24.8 / 19.6 / 19.1 (imaginary time
+//     17.7 / 18.6)
+int patch_cells(const ts_b200_kernel *k) {
+    if (!k->patch || k->walk2 != 2) return 0;
+    int most2, most4;  // regions
+    if ((k->phase & 3) == 3) {
+        most2 = k->fp32 ? 256 : 1100;
+        most4 = k->fp32 ? 400 : 0;
+    } else if (k->rot) {
+        most2 = 320;
+        most4 = k->fp32 ? 2000 : 870;
+    } else if (k->cyl) {
+        most2 = 260;
+        most4 = k->fp32 ? 1100 : 300;
+    } else {
+        most2 = k->fp32 ? 1100 : 2100;
+        most4 = k->fp32 ? (k->imag ? 900 : 600) : 0;
+    }
+    int nx, ny;
+    if (patch_regions(k, 2, &nx, &ny) <= most2) return 2;
+    if (patch_regions(k, 4, &nx, &ny) <= most4) return 4;
+    return 0;
+}
+
+// Grid of the patch step: the regions, taken in turn by the blocks that the
+// GPU holds.
+void patch_geometry(const ts_b200_kernel *k, int n, int *nx, int *ny, int *blocks) {
+    *blocks = std::min(patch_regions(k, n, nx, ny), tsb::patch_blocks(n, k->fp32) * k->num_sms);
+}
+
+// Programmatic dependent launch of a step.  Patches: not between half a block
+// and two blocks per SM, where the next step's blocks share SMs with this
+// step's while others idle (121 blocks: rotating frame 512^2 10.7 -> 13.8 us;
+// 9 blocks: 3.5 -> 3.3, 444 blocks: 7.2 -> 6.8); always with potential rows,
+// whose steps are queued one by one (256^2 6.5 -> 5.3).
+bool step_pdl(const ts_b200_kernel *k, int patch, int blocks) {
+    if (!patch || k->overlap_set) return walk_pdl(k);
+    return k->vpot || 2 * blocks <= k->num_sms || blocks >= 2 * k->num_sms;
+}
+
+template <typename T>
+cudaError_t launch_patch(const ts_b200_kernel *k, int n, int phase, StepArgs<T> &a, int blocks,
+                         cudaStream_t st, bool pdl) {
+    if (k->wrap_next) {
+        a.wrap = (k->d.periodic_x ? 1 : 0) | (k->d.periodic_y ? 2 : 0);
+        a.wrap_hx = k->d.halo_x;
+        a.wrap_hy = k->d.halo_y;
+        a.wrap_y0 = k->d.inner_y0;
+        a.wrap_y1 = k->d.inner_y0 + k->H - 2 * k->d.halo_y;
+    }
+    if constexpr (sizeof(T) == 8)
+        return k->imag ? tsb::launch_patch_f64_imag(n, k->rot, phase, a, blocks, st, pdl)
+                       : tsb::launch_patch_f64_real(n, k->rot, phase, a, blocks, st, pdl);
+    else
+        return k->imag ? tsb::launch_patch_f32_imag(n, k->rot, phase, a, blocks, st, pdl)
+                       : tsb::launch_patch_f32_real(n, k->rot, phase, a, blocks, st, pdl);
+}
+
 // Resident blocks of this variant and shape (the persistent grid size) and,
 // from them, the segment height.
 template <typename T>
@@ -831,6 +924,9 @@ int launch_step_buffers_t(ts_b200_kernel *k, const void *in, void *out, bool dry
     const int c = configure_t<T>(k);
     if (c) return c;
     geometry(k, &strips, &segs, &blocks, &smem);
+    const int patch = patch_cells(k);
+    if (patch) patch_geometry(k, patch, &strips, &segs, &blocks);
+    const bool pdl = step_pdl(k, patch, blocks);
     const size_t nwarps = (size_t)std::max(blocks, 1) * k->warps;
     if (k->imag && nwarps > k->partials_cap) {
         if (k->partials) cudaFree(k->partials);
@@ -856,8 +952,10 @@ int launch_step_buffers_t(ts_b200_kernel *k, const void *in, void *out, bool dry
         a.pot_dt = k->vpot_dt;
         phase |= 16;
     }
-    cudaError_t e = dispatch_step<T>(k->C, k->imag, k->rot, phase, walk_rows(k), a, k->warps,
-                                     smem, blocks, k->stream, nullptr, k->overlap);
+    cudaError_t e =
+        patch ? launch_patch<T>(k, patch, phase, a, blocks, k->stream, pdl)
+              : dispatch_step<T>(k->C, k->imag, k->rot, phase, walk_rows(k), a, k->warps, smem,
+                                 blocks, k->stream, nullptr, pdl);
     if (e != cudaSuccess) return cuda_fail(k, e, "step kernel launch");
     if (!dry) g_launches.fetch_add(1, std::memory_order_relaxed);
     return TS_B200_OK;
@@ -868,10 +966,11 @@ int launch_step_t(ts_b200_kernel *k, int exchange, bool dry = false) {
     const int s = launch_step_buffers_t<T>(k, k->psi[k->cur], k->psi[1 - k->cur], dry);
     if (s || dry) return s;
     k->cur = 1 - k->cur;
-    if (exchange) {
+    if (exchange && !k->wrap_steps) {
         const int st = launch_halo_t<T>(k);
         if (st) return st;
     }
+    k->wrap_next = exchange && k->wrap_steps;
     return TS_B200_OK;
 }
 
@@ -886,10 +985,16 @@ int launch_step_part_t(ts_b200_kernel *k, const void *in, void *out, const tsbh:
     if (p.a1 > 0 && (p.a0 < 0 || p.a1 <= p.a0 || p.a1 > k->H || (p.a0 & 1) ||
                      (p.b1 > p.b0 && (p.b0 < 0 || p.b1 > k->H || (p.b0 & 1)))))
         return fail(k, TS_B200_INVALID_ARGUMENT, "step part: row windows");
-    const bool pdl = p.pdl && p.a1 == 0 && k->overlap && use_walk2(k);
+    bool pdl = p.pdl && p.a1 == 0 && walk_pdl(k) && use_walk2(k);
     int strips, segs, blocks;
     size_t smem;
     geometry(k, &strips, &segs, &blocks, &smem, pdl, &p);
+    const int patch = p.a1 == 0 ? patch_cells(k) : 0;
+    if (patch) {
+        patch_geometry(k, patch, &strips, &segs, &blocks);
+        if (p.blocks > 0) blocks = std::min(blocks, p.blocks);
+        pdl = p.pdl && step_pdl(k, patch, blocks);
+    }
     double *partials = p.partials;
     if (k->imag && !partials) {
         const size_t nb = (size_t)std::max(blocks, 1);
@@ -923,8 +1028,10 @@ int launch_step_part_t(ts_b200_kernel *k, const void *in, void *out, const tsbh:
     a.pair_norm = p.pair_norm;
     a.pair_ticket = p.pair_ticket;
     a.pair_slot = p.pair_slot;
-    cudaError_t e = dispatch_step<T>(k->C, k->imag, k->rot, k->phase, walk_rows(k), a, k->warps,
-                                     smem, blocks, p.stream ? p.stream : k->stream, nullptr, pdl);
+    const cudaStream_t st = p.stream ? p.stream : k->stream;
+    cudaError_t e = patch ? launch_patch<T>(k, patch, k->phase, a, blocks, st, pdl)
+                          : dispatch_step<T>(k->C, k->imag, k->rot, k->phase, walk_rows(k), a,
+                                             k->warps, smem, blocks, st, nullptr, pdl);
     if (e != cudaSuccess) return cuda_fail(k, e, "step part launch");
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TS_B200_OK;
@@ -940,6 +1047,11 @@ int tsbh::part_blocks(const ts_b200_kernel *k, const tsbh::StepPart &p) {
     int strips, segs, blocks;
     size_t smem;
     geometry(k, &strips, &segs, &blocks, &smem, false, &p);
+    const int patch = p.a1 == 0 ? patch_cells(k) : 0;
+    if (patch) {
+        patch_geometry(k, patch, &strips, &segs, &blocks);
+        if (p.blocks > 0) blocks = std::min(blocks, p.blocks);
+    }
     return std::max(blocks, 1);
 }
 
@@ -974,7 +1086,7 @@ int tsbh::launch_step_buffers(ts_b200_kernel *k, const void *in, void *out) {
 namespace {
 
 int kernels_per_step(const ts_b200_kernel *k, int exchange) {
-    return 1 + ((exchange && (k->d.periodic_x || k->d.periodic_y)) ? 1 : 0);
+    return 1 + ((exchange && (k->d.periodic_x || k->d.periodic_y) && !k->wrap_steps) ? 1 : 0);
 }
 
 int check_device_error(ts_b200_kernel *k) {
@@ -1507,7 +1619,17 @@ int ts_b200_evolve(ts_b200_kernel *k, int iterations) {
     // the buffers as it found them).
     const int G = 32;
     int remaining = iterations - 1;  // exchanging steps
-    if (remaining > 0 && k->cur != 0) {
+    // The patch step reads the halo of the previous step's output from the
+    // cells the refresh would copy (no refresh launch): every step but the
+    // first; the last step's output keeps its own halo, as without it.
+    k->wrap_steps = (k->d.periodic_x || k->d.periodic_y) && patch_cells(k) > 0;
+    struct Reset {
+        ts_b200_kernel *k;
+        ~Reset() { k->wrap_steps = k->wrap_next = false; }
+    } reset{k};
+    // plain steps up to buffer 0 and, with wrapped steps, past the first one
+    // (the graph's first step wraps)
+    while (remaining > 0 && (k->cur != 0 || (k->wrap_steps && !k->wrap_next))) {
         int s = launch_step(k, 1);
         if (s) return s;
         --remaining;
@@ -1675,6 +1797,21 @@ int ts_b200_launch_info(const ts_b200_kernel *k, ts_b200_launch_shape *out) {
     int strips, segs, blocks;
     size_t smem;
     geometry(k, &strips, &segs, &blocks, &smem);
+    if (const int n = patch_cells(k)) {
+        patch_geometry(k, n, &strips, &segs, &blocks);
+        const bool all_rows = k->rot || k->cyl;
+        *out = ts_b200_launch_shape{};
+        out->cells_per_lane = n;
+        out->segment_rows = tsb::patch_out(n, k->rot ? 6 : 4);
+        out->warps_per_block = 8;
+        out->strips = strips;
+        out->segments = segs;
+        out->blocks = blocks;
+        out->threads = 256;
+        out->smem_bytes = (int64_t)2 * (all_rows ? n : n / 2) * 256 * k->cell;
+        out->walk = 3;
+        return TS_B200_OK;
+    }
     out->cells_per_lane = k->C;
     out->segment_rows = eff_seg(k);
     out->warps_per_block = k->warps;
@@ -1705,6 +1842,7 @@ int ts_b200_set_launch(ts_b200_kernel *k, int C, int seg_h, int warps, int ring)
     if (ring != 0 && (ring < min_ring(k) || ring > 16))
         return fail(k, TS_B200_INVALID_ARGUMENT, "ring depth out of range for this variant");
     if (seg_h < 0) return TS_B200_INVALID_ARGUMENT;
+    k->patch = false;
     if (C) k->C = C;
     if (seg_h) {
         k->seg_h = seg_h;
@@ -1723,6 +1861,8 @@ int ts_b200_set_launch(ts_b200_kernel *k, int C, int seg_h, int warps, int ring)
 
 int ts_b200_set_walk(ts_b200_kernel *k, int walk) {
     if (!k || walk < 0 || walk > 2) return TS_B200_INVALID_ARGUMENT;
+    if (k->patch) drop_graph(k);
+    k->patch = false;
     if (k->walk2 == walk) return TS_B200_OK;
     k->walk2 = walk;
     if (!use_walk2(k) && k->warps > 4) k->warps = 4;
@@ -1735,8 +1875,9 @@ int ts_b200_set_walk(ts_b200_kernel *k, int walk) {
 
 int ts_b200_set_overlap(ts_b200_kernel *k, int on) {
     if (!k || (on != 0 && on != 1)) return TS_B200_INVALID_ARGUMENT;
-    if (k->overlap != (on == 1)) {
+    if (k->overlap != (on == 1) || !k->overlap_set) {
         k->overlap = on == 1;
+        k->overlap_set = true;
         drop_graph(k);
     }
     return TS_B200_OK;
@@ -1752,14 +1893,34 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
     TSB_CHECK(k, cudaMemcpyAsync(&saved, k->scal, sizeof saved, cudaMemcpyDeviceToHost, k->stream));
     TSB_CHECK(k, cudaStreamSynchronize(k->stream));
     const int C0 = k->C, seg0 = k->seg_h, warps0 = k->warps;
-    const bool auto0 = k->auto_seg, overlap0 = k->overlap;
+    const bool auto0 = k->auto_seg, overlap0 = k->overlap, overlap_set0 = k->overlap_set;
+    const bool patch0 = k->patch;
     cudaEvent_t e0, e1;
     TSB_CHECK(k, cudaEventCreate(&e0));
     TSB_CHECK(k, cudaEventCreate(&e1));
     float best_ms = -1.0f;
     int best_seg = seg0, best_warps = warps0;
-    bool best_overlap = overlap0;
+    bool best_overlap = overlap0, best_patch = false;
     int st = TS_B200_OK;
+    // trial_steps steps of the current choice, after one untimed
+    auto time_steps = [&](float *ms) {
+        int s = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
+        if (s) return s;
+        cudaEventRecord(e0, k->stream);
+        for (int i = 0; i < trial_steps && s == TS_B200_OK; ++i)
+            s = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
+        cudaEventRecord(e1, k->stream);
+        cudaError_t e = cudaEventSynchronize(e1);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
+        if (s == TS_B200_OK && e != cudaSuccess) s = cuda_fail(k, e, "autotune timing");
+        return s;
+    };
+    // the register patches, where they are this tile's default
+    if (patch_cells(k)) {
+        st = time_steps(&best_ms);
+        best_patch = st == TS_B200_OK;
+    }
+    k->patch = false;
     // the look-ahead walk: blocks of 4 or 8 warps (4 or 2 in a rotating
     // frame), with and without programmatic dependent launch; the checked
     // walk: 4 or 2 warps
@@ -1768,6 +1929,7 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
     for (int trial = 0; trial < (w2 ? 4 : 2) && st == TS_B200_OK; ++trial) {
         const int warps = warp_opts[trial & 1];
         k->overlap = w2 ? ((trial >> 1) ? !overlap0 : overlap0) : overlap0;
+        k->overlap_set = true;
         k->warps = warps;
         k->resident_blocks = 0;
         k->auto_seg = false;
@@ -1786,21 +1948,12 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
             for (int d = 0; d < c; ++d) seen = seen || cand[d] == cand[c];
             if (seen) continue;
             k->seg_h = cand[c];
-            st = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
-            if (st) break;
-            cudaEventRecord(e0, k->stream);
-            for (int i = 0; i < trial_steps && st == TS_B200_OK; ++i)
-                st = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
-            cudaEventRecord(e1, k->stream);
-            cudaError_t e = cudaEventSynchronize(e1);
             float ms = 0.0f;
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-            if (e != cudaSuccess) {
-                st = cuda_fail(k, e, "autotune timing");
-                break;
-            }
+            st = time_steps(&ms);
+            if (st) break;
             if (best_ms < 0.0f || ms < best_ms) {
                 best_ms = ms;
+                best_patch = false;
                 best_seg = k->seg_h;
                 best_warps = warps;
                 best_overlap = k->overlap;
@@ -1810,21 +1963,22 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (st) {
-        k->C = C0;
+    k->C = C0;
+    k->resident_blocks = 0;
+    if (st || best_patch) {
         k->seg_h = seg0;
         k->warps = warps0;
         k->auto_seg = auto0;
         k->overlap = overlap0;
-        k->resident_blocks = 0;
-        return st;
+        k->overlap_set = overlap_set0;
+        k->patch = patch0;
+        if (st) return st;
+    } else {
+        k->seg_h = best_seg;
+        k->warps = best_warps;
+        k->overlap = best_overlap;
+        k->auto_seg = false;
     }
-    k->C = C0;
-    k->seg_h = best_seg;
-    k->warps = best_warps;
-    k->overlap = best_overlap;
-    k->auto_seg = false;
-    k->resident_blocks = 0;
     drop_graph(k);
     TSB_CHECK(k, cudaMemcpyAsync(k->scal, &saved, sizeof saved, cudaMemcpyHostToDevice, k->stream));
     TSB_CHECK(k, cudaStreamSynchronize(k->stream));

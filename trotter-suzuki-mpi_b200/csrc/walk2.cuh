@@ -758,9 +758,11 @@ __device__ __forceinline__ void w2_task(Walk2<V, R> &w, const StepArgs<typename 
 // last block advances the coefficient schedule; in imaginary time the block
 // partials of the squared norm are summed in a fixed order by the last block,
 // which sets the renormalisation factor the next step applies.
+// scratch: kFinishScratch doubles of shared memory (imaginary time).
+constexpr int kFinishScratch = 65;
 template <class V>
 __device__ __forceinline__ void w2_finish(const StepArgs<typename V::T> &a, double nacc, int warps,
-                                          int warp, int lane) {
+                                          int warp, int lane, double *scratch) {
     if constexpr (!V::IMAG && DeltaForm<typename V::T>::value) {
         if (a.kin_sched) {
             __syncthreads();
@@ -778,9 +780,8 @@ __device__ __forceinline__ void w2_finish(const StepArgs<typename V::T> &a, doub
     if constexpr (V::IMAG) {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) nacc += __shfl_xor_sync(0xffffffffu, nacc, off);
-        __shared__ double s_warp[32];
-        __shared__ unsigned int s_last;
-        __shared__ double red[32];
+        double *s_warp = scratch, *red = scratch + 32;
+        unsigned int &s_last = *reinterpret_cast<unsigned int *>(scratch + 64);
         if (lane == 0) s_warp[warp] = nacc;
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -957,7 +958,8 @@ __global__ void __launch_bounds__(W2Bounds<V>::THREADS, W2Bounds<V>::MIN_BLOCKS)
          task += gridDim.x * warps)
         w2_task(w, a, task);
 
-    w2_finish<V>(a, w.nacc, warps, warp, lane);
+    __shared__ double s_finish[V::IMAG ? kFinishScratch : 1];
+    w2_finish<V>(a, w.nacc, warps, warp, lane, s_finish);
 }
 
 // Many tiles of one precision and time mode in one persistent launch (the
