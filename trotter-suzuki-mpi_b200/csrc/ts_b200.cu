@@ -652,16 +652,36 @@ int balanced_segments(const ts_b200_kernel *k, int blocks_per_sm, int warps) {
     return use_walk2(k) ? (seg + 1) & ~1 : seg;
 }
 
-// Default: 4 blocks of 4 warps per SM (fewer, taller tasks than a grid
-// filling every resident slot: less halo work per row, the same balance),
-// with segments of at most kMaxAutoSegment rows: on large tiles one task per
+// Default: one task per warp with 1 .. 4 blocks of 4 warps per SM.  More
+// warps share the latency of the row chain, but their shorter segments walk
+// more halo rows (2 HY per segment): the walked rows times what a row costs
+// with b blocks on the SM is smallest.  The costs are the times per walked
+// row at 1200^2 .. 2500^2 (double, imaginary time 0.43 / 0.57 / 0.74 / 0.92 us
+// with 1 .. 4 blocks, float 0.33 / 0.42 / 0.53 / 0.66, double cylinder 0.58 /
+// 0.75 / 0.98 / 1.26; rotating frame, double 0.85 / 0.93 / 1.20).  Against 4
+// blocks everywhere: cylinder 1024^2 23.2 -> 21.3 us, 1500^2 34.7 -> 32.4,
+// double 1300^2 21.5 -> 20.1, float 1800^2 22.1 -> 21.6; 2048^2 keeps 4.
+// Segments have at most kMaxAutoSegment rows: on large tiles one task per
 // warp means segments of hundreds of rows, which ran 1.3-1.6x slower than
 // 64-128-row segments taken by the persistent warps in turn (8192^2 rotating
 // frame: 2.02 -> 1.35 ms per step in double, 1.72 -> 1.07 in float).
 constexpr int kMaxAutoSegment = 128;
 void auto_segments(ts_b200_kernel *k) {
-    const int bps = std::max(1, k->resident_blocks / std::max(1, k->num_sms));
-    k->seg_h = std::min(kMaxAutoSegment, balanced_segments(k, std::min(4, bps), k->warps));
+    static const double cost[2][4] = {{1.0, 1.32, 1.70, 2.13}, {1.0, 1.09, 1.42, 2.30}};
+    const int bps = std::min(4, std::max(1, k->resident_blocks / std::max(1, k->num_sms)));
+    const bool walk2 = use_walk2(k);
+    double best = 0.0;
+    k->seg_h = kMaxAutoSegment;
+    for (int b = bps; b >= 1; --b) {
+        const int seg = balanced_segments(k, b, k->warps);
+        // the checked walk keeps the most blocks
+        if (seg > kMaxAutoSegment || (b < bps && !walk2)) break;
+        const double c = (seg + 2 * (k->rot ? 6 : 4)) * cost[k->rot][b - 1];
+        if (b == bps || c < best) {
+            best = c;
+            k->seg_h = seg;
+        }
+    }
 }
 
 // Programmatic dependent launch of a row walk's steps: where it was asked for
@@ -776,18 +796,9 @@ void tsbh::fill_step_constants(const ts_b200_kernel *k, StepArgs<T> &a) {
         const double ky = k->imag ? asinh(k->d.b_v) : asin(k->d.b_v);
         const double amh = k->imag ? cosh_m1(kx) : cos_m1(kx);
         const double amv = k->imag ? cosh_m1(ky) : cos_m1(ky);
-        float fa, fb;
-        if (k->imag) {
-            a.aH = (T)amh;
-            a.aV = (T)amv;
-        } else {
-            unimodular_float_pair(amh, k->d.b_h, 16, &fa, &fb);
-            a.aH = (T)fa;
-            a.bH = (T)fb;
-            unimodular_float_pair(amv, k->d.b_v, 16, &fa, &fb);
-            a.aV = (T)fa;
-            a.bV = (T)fb;
-        }
+        // real time: replaced by the step's entry of the coefficient schedule
+        a.aH = (T)amh;
+        a.aV = (T)amv;
     }
     a.ca = (T)k->d.coupling;
     a.caa = (T)k->d.lhy_coupling;
@@ -826,35 +837,37 @@ int patch_regions(const ts_b200_kernel *k, int n, int *nx, int *ny) {
 // are the region counts up to which each was the fastest of the three on
 // square tiles (us per step, 2 x 2 / 4 x 4 / walk):
 //   double, 4 halo columns: 256^2 3.3 / 8.4 / 9.3, 512^2 6.2 / 8.7 / 10.9,
-//     1024^2 15.1 / 18.8 / 18.2, 1280^2 26.0 / 23.6 / 21.5; imaginary time
-//     1024^2 17.3 / 19.0 / 18.8; potential rows 1024^2 19.2 / 28.0 / 24.9
-//   one species of a pair: 768^2 18.0 / 21.0 / 19.4, 1024^2 26.7 / 34.5 / 24.1;
-//     float 1024^2 20.3 / 17.6 / 18.9
-//   rotating frame, double: 256^2 5.8 / 10.1 / 18.9, 512^2 13.3 / 10.6 / 20.7,
-//     1024^2 41.7 / 25.6 / 32.0, 1300^2 - / 40.3 / 41.6
-//   rotating frame, float: 256^2 6.6 / 9.4 / 26.3, 512^2 11.0 / 9.8 / 26.5,
-//     2048^2 96.1 / 47.6 / 59.9, 4096^2 388 / 171 / 152
-//   cylinder, double: 256^2 7.7 / 11.0 / 12.7, 512^2 13.3 / 12.2 / 14.3,
-//     768^2 21.0 / 15.8 / 17.1, 1024^2 32.1 / 26.2 / 24.6
+//     1024^2 15.0 / 18.8 / 16.9, 1280^2 26.0 / 23.6 / 20; imaginary time
+//     1024^2 17.2 / 19.0 / 16.8, linear 13.7 / - / 12.8; potential rows 18.0 /
+//     28.0 / 20.7
+//   one species of a pair: 640^2 12.8 / - / 14.3, 768^2 17.8 / 21.0 / 15.7;
+//     float 512^2 8.9 / 13.0 / 11.6, 640^2 12.2 / 13.2 / 11.6
+//   rotating frame, double: 256^2 5.9 / 10.1 / 18.8, 512^2 13.3 / 10.6 / 20.6,
+//     1024^2 41.7 / 26.2 / 32.1, 1300^2 - / 41.0 / 42.3
+//   rotating frame, float: 256^2 6.6 / 9.4 / 25.2, 512^2 11.0 / 9.9 / 25.8,
+//     2048^2 96.1 / 48.4 / 54.4, 4096^2 388 / 171 / 152
+//   cylinder, double: 256^2 7.9 / 11.0 / 12.8, 512^2 13.3 / 11.8 / 13.9,
+//     830^2 - / 15.1 / 17.7, 1024^2 32.1 / 26.2 / 21.3
 //   cylinder, float: 512^2 9.8 / 9.1 / 11.4, 1536^2 39.6 / 23.2 / 24.1
 //   float, 4 halo columns: 512^2 6.5 / 8.1 / 9.2, 768^2 9.1 / 10.1 / 10.5,
-//     1024^2 13.3 / 11.7 / 13.8, 1536^2 24.8 / 19.6 / 19.1 (imaginary time
-//     17.7 / 18.6)
+//     1024^2 13.3 / 11.9 / 13.1, 1280^2 - / 16.2 / 15.0 (imaginary time 1536^2
+//     - / 17.8 / 18.2)
 int patch_cells(const ts_b200_kernel *k) {
     if (!k->patch || k->walk2 != 2) return 0;
-    int most2, most4;  // regions
+    int most2, most4 = 0;  // regions
     if ((k->phase & 3) == 3) {
-        most2 = k->fp32 ? 256 : 1100;
-        most4 = k->fp32 ? 400 : 0;
+        most2 = k->fp32 ? 520 : 750;
     } else if (k->rot) {
         most2 = 320;
         most4 = k->fp32 ? 2000 : 870;
     } else if (k->cyl) {
         most2 = 260;
         most4 = k->fp32 ? 1100 : 300;
+    } else if (k->fp32) {
+        most2 = 1100;
+        most4 = k->imag ? 900 : 430;
     } else {
-        most2 = k->fp32 ? 1100 : 2100;
-        most4 = k->fp32 ? (k->imag ? 900 : 600) : 0;
+        most2 = (k->imag || k->phase == 0) ? 1600 : 2100;
     }
     int nx, ny;
     if (patch_regions(k, 2, &nx, &ny) <= most2) return 2;
