@@ -519,7 +519,10 @@ __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 // 43.9-48.0 (phases of the second tier 46.6 / 49.7, of the library 65.2 /
 // 63.6).  Float gains nothing by it (25.5 / 25.9; library 47.7 / 43.7) and
 // nor does the double rotating frame (2048^2 74.7 / 73.6), which keep the
-// warp's choice.  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
+// warp's choice.  REST: all but the first tier in a function of its own, for
+// the float rotating frame, whose row body is bound by instruction fetch
+// (4096^2 151.3 -> 143.2 us, 2300^2 67.6 -> 62.9; phases of the second tier
+// 154.1 -> 164.4, of the library 225 -> 234).  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
 // The comparisons are exact in either precision.
 __device__ __forceinline__ bool phase_tiny(double th) { return fabs(th) < 0.00390625; }
 __device__ __forceinline__ bool phase_tiny(float th) { return fabsf(th) < 0.00390625f; }
@@ -575,12 +578,21 @@ __device__ __forceinline__ void sincos_large(T th, T *s, T *c) {
     }
 }
 
+template <typename T>
+static __device__ __noinline__ void sincos_rest(T th, T *s, T *c) {
+    if (!__any_sync(0xffffffffu, !phase_small(th))) sincos_small(th, s, c);
+    else sincos_large(th, s, c);
+}
+
 // TIERS = false: the 1/32 tier and the library only (less code, for the
 // kernels whose row body is long enough for instruction fetch to limit them).
-template <typename T, bool TIERS = true, bool CELL = std::is_same<T, double>::value>
+template <typename T, bool TIERS = true, bool CELL = std::is_same<T, double>::value,
+          bool REST = false>
 __device__ __forceinline__ void phase_sincos(T th, T *s, T *c) {
     if (TIERS && !__any_sync(0xffffffffu, !phase_tiny(th))) {
         sincos_tiny(th, s, c);
+    } else if (REST) {
+        sincos_rest(th, s, c);
     } else if (CELL) {
         sincos_small(th, s, c);
         if (TIERS && phase_tiny(th)) sincos_tiny(th, s, c);
@@ -791,7 +803,8 @@ __device__ __forceinline__ void potential_row(Cx<T> (&w)[C], const TabT *tab, T 
                 T th = mul_t(ca, n2);
                 if (LHY) th = fma_t(caa, mul_t(n2, sqrt_t(n2)), th);
                 if (PB) th = th + thb;
-                phase_sincos<T, TIERS, std::is_same<T, double>::value && !ROT>(th, &s, &c);
+                constexpr bool F32 = std::is_same<T, float>::value;
+                phase_sincos<T, TIERS, !F32 && !ROT, F32 && ROT>(th, &s, &c);
             }
             // the table holds (cos, sin) of -dt V; in delta form (cos - 1, sin):
             // v (cos + i sin), the kinetic pair's form with the cell as its own
