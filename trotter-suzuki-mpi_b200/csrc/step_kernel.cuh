@@ -518,11 +518,12 @@ __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 // across them: the 2048^2 double real-time step took 38.7 us against
 // 43.9-48.0 (phases of the second tier 46.6 / 49.7, of the library 65.2 /
 // 63.6).  Float gains nothing by it (25.5 / 25.9; library 47.7 / 43.7) and
-// nor does the double rotating frame (2048^2 74.7 / 73.6), which keep the
-// warp's choice.  REST: all but the first tier in a function of its own, for
-// the float rotating frame, whose row body is bound by instruction fetch
-// (4096^2 151.3 -> 143.2 us, 2300^2 67.6 -> 62.9; phases of the second tier
-// 154.1 -> 164.4, of the library 225 -> 234).  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
+// keeps the warp's choice.  REST: that choice with all but the first tier in
+// a function of its own, for the rotating frame, whose row body is bound by
+// instruction fetch (float 4096^2 151.3 -> 143.2 us, 2300^2 67.6 -> 62.9,
+// double 1400^2 46.1 -> 44.0, 2048^2 76.6 -> 75.5, 4096^2 291.8 -> 288.5, 3000^2
+// 140.2 -> 142; float with phases of the second tier 154.1 -> 164.4, of the
+// library 225 -> 234).  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
 // The comparisons are exact in either precision.
 __device__ __forceinline__ bool phase_tiny(double th) { return fabs(th) < 0.00390625; }
 __device__ __forceinline__ bool phase_tiny(float th) { return fabsf(th) < 0.00390625f; }
@@ -804,7 +805,7 @@ __device__ __forceinline__ void potential_row(Cx<T> (&w)[C], const TabT *tab, T 
                 if (LHY) th = fma_t(caa, mul_t(n2, sqrt_t(n2)), th);
                 if (PB) th = th + thb;
                 constexpr bool F32 = std::is_same<T, float>::value;
-                phase_sincos<T, TIERS, !F32 && !ROT, F32 && ROT>(th, &s, &c);
+                phase_sincos<T, TIERS, !F32 && !ROT, ROT>(th, &s, &c);
             }
             // the table holds (cos, sin) of -dt V; in delta form (cos - 1, sin):
             // v (cos + i sin), the kinetic pair's form with the cell as its own
