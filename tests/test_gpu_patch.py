@@ -177,6 +177,34 @@ def test_patches_with_potential_rows(W, H, pad):
     assert np.array_equal(out[None], out[0])
 
 
+@pytest.mark.parametrize("N,Ny", [(1, 1), (24, 24), (25, 49), (131, 90)])
+@pytest.mark.parametrize("g,lhy,every,imag", [(0.0, 0.0, 0, False), (8.0, 0.0, 4, False),
+                                              (8.0, 0.5, 3, False), (0.0, 0.0, 5, True),
+                                              (8.0, 0.5, 4, True)])
+def test_adjoint_patches_match_the_row_walk(N, Ny, g, lhy, every, imag):
+    """Gradients of 10 steps: the row walk's bits in real time; in imaginary
+    time the inner products are summed over another grid of blocks."""
+    import torch
+    from trottersuzuki_b200.adjoint import AdjointEngine
+    lat, psi0, V = seeded_case(N, 10.0 if N > 1 else 1.0, Ny)
+    n0 = O.expectations(lat, psi0)["norm2"] if imag else 0.0
+    p = lat.params(1e-3, imag, 1.0, g, lhy, norm0=n0)
+    v = torch.tensor(V, device="cuda")
+    psi = torch.tensor(psi0, device="cuda")
+    lam = torch.randn(psi.shape, dtype=torch.complex128, device="cuda",
+                      generator=torch.Generator("cuda").manual_seed(3))
+    out = []
+    for rows in (0, 6):
+        e = AdjointEngine(desc_from_params(p), 1e-3, 10, every)
+        if rows:
+            e.set_segments(adjoint_rows=rows)
+        e.forward(v, psi)
+        out.append([t.cpu().numpy() for t in e.backward(lam)])
+        e.close()
+    for got, old in zip(*out):
+        _close(got, old, imag)
+
+
 def test_asking_for_a_walk_or_overlap_after_steps_keeps_the_evolution():
     """Switches of walk and launch mode between evolve calls that replay graphs."""
     from trottersuzuki_b200 import Kernel

@@ -23,6 +23,7 @@
 #include <string>
 
 #include "adjoint_kernel.cuh"
+#include "adjoint_patch_decl.h"
 #include "handle.h"
 #include "ts_b200.h"
 
@@ -42,6 +43,7 @@ struct ts_b200_adjoint {
     void *ckpt = nullptr;  // n_ckpt states
     int *error = nullptr;
     int seg_h = 32, warps = 2, ring = 4, blocks = 0;
+    bool patch = true;  // register patches where they are faster; off once segments were asked for
     bool forward_done = false;
     // imaginary time: factors c of the checkpoints and of a segment's states,
     // the projection coefficients mu (ping-pong), the running sum of the
@@ -238,6 +240,39 @@ cudaError_t launch_adj(ts_b200_adjoint *a, int mode, int phase, const AdjArgs &a
     return launch_adj_variant<AdjVariant<1, 0>>(a, args, blocks, bps);
 }
 
+// Regions of the pass on register patches, 0 where the row walk takes it: on
+// large tiles, and where its segments were asked for (us per step of the
+// reverse pass, patches / walk; linear 256^2 4.8 / 18.5, 512^2 10.5 / 21.3,
+// 900^2 23.5 / 28.9, 1024^2 34.4 / 32.0; checkpointed GPE 512^2 13.3 / 32.6,
+// 1024^2 44.3 / 54.4, 1280^2 80.5 / 74.4; imaginary time 512^2 18.7 / 33.6,
+// 1024^2 49.1 / 52.7, 1280^2 73.8 / 64.2).
+int adj_patch_regions(const ts_b200_adjoint *a) {
+    constexpr int out = tsb::patch_out(tsb::kAdjPatch, AdjVariant<0, 0>::HX);
+    const long n = (long)div_up(a->W, out) * div_up(a->H, out);
+    return a->patch && n <= (a->every > 0 ? 1900 : 1500) ? (int)n : 0;
+}
+
+// One pass with the arguments of its fields.
+int launch_pass(ts_b200_adjoint *a, int mode, AdjArgs &x) {
+    cudaError_t e;
+    if (const int n = adj_patch_regions(a)) {
+        constexpr int out = tsb::patch_out(tsb::kAdjPatch, AdjVariant<0, 0>::HX);
+        x.n_strips = div_up(a->W, out);
+        x.n_segs = div_up(a->H, out);
+        const int blocks = std::min(n, tsb::kAdjPatchBlocks * a->k->num_sms);
+        // as for the patches of a step (step_pdl)
+        const bool pdl = 2 * blocks <= a->k->num_sms || blocks >= 2 * a->k->num_sms;
+        e = tsb::launch_adj_patch(mode, a->k->phase, x, blocks, a->k->stream, pdl);
+    } else {
+        const int tasks = x.n_strips * x.n_segs;
+        const int blocks = std::max(1, std::min(a->blocks, div_up(tasks, a->warps)));
+        e = launch_adj(a, mode, a->k->phase, x, blocks, nullptr);
+    }
+    if (e != cudaSuccess) return acuda(a, e, "adjoint kernel launch");
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TS_B200_OK;
+}
+
 AdjArgs adj_args(ts_b200_adjoint *a) {
     const ts_b200_desc &d = a->k->d;
     AdjArgs x{};
@@ -282,12 +317,7 @@ int adj_step_imag(ts_b200_adjoint *a, const void *psi_k_in, const double *c_k, c
     x.mu_next = mu_in;
     x.mu_out = mu_out;
     x.accumulate = accumulate ? 1 : 0;
-    const int tasks = x.n_strips * x.n_segs;
-    const int blocks = std::max(1, std::min(a->blocks, div_up(tasks, a->warps)));
-    cudaError_t e = launch_adj(a, 2, a->k->phase, x, blocks, nullptr);
-    if (e != cudaSuccess) return acuda(a, e, "adjoint kernel launch");
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return TS_B200_OK;
+    return launch_pass(a, 2, x);
 }
 
 int adj_step(ts_b200_adjoint *a, int mode, const void *psi_in, void *psi_out, const void *lam_in,
@@ -297,12 +327,7 @@ int adj_step(ts_b200_adjoint *a, int mode, const void *psi_in, void *psi_out, co
     x.psi_out = psi_out;
     x.lam_in = lam_in;
     x.lam_out = lam_out;
-    const int tasks = x.n_strips * x.n_segs;
-    const int blocks = std::max(1, std::min(a->blocks, div_up(tasks, a->warps)));
-    cudaError_t e = launch_adj(a, mode, a->k->phase, x, blocks, nullptr);
-    if (e != cudaSuccess) return acuda(a, e, "adjoint kernel launch");
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    return TS_B200_OK;
+    return launch_pass(a, mode, x);
 }
 
 int tile_status(ts_b200_adjoint *a, int s) {
@@ -574,7 +599,8 @@ int ts_b200_adjoint_set_segments(ts_b200_adjoint *a, int adjoint_rows, int forwa
         if (s) return s;
         drop_segment_graphs(a);
     }
-    if (adjoint_rows > 0 && adjoint_rows != a->seg_h) {
+    if (adjoint_rows > 0 && (a->patch || adjoint_rows != a->seg_h)) {
+        a->patch = false;
         a->seg_h = adjoint_rows;
         if (a->inv_graph) cudaGraphExecDestroy(a->inv_graph);
         a->inv_graph = nullptr;

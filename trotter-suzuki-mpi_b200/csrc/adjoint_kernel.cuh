@@ -94,7 +94,8 @@ struct AdjVariant {
     // slot: psi | lambda | [psi_{k+1}] | table | dL/dV
     static constexpr int PSN_OFF = 2 * ROW;
     static constexpr int TAB_OFF = IMAG ? 3 * ROW : 2 * ROW;
-    static constexpr int TAB_CELL = IMAG ? 8 : 16;  // real table in imaginary time
+    using TabT = typename std::conditional<IMAG, double, Cx<double>>::type;
+    static constexpr int TAB_CELL = (int)sizeof(TabT);  // real table in imaginary time
     static constexpr int GV_OFF = TAB_OFF + SW * TAB_CELL;
     static constexpr int SLOT = GV_OFF + SW * 8;
 };
@@ -146,87 +147,77 @@ __device__ __forceinline__ void adj_h(AdjWalk &w, Cx<double> (&row)[2]) {
     hsweep_lane<IM, PAR>(row, w.hai, s * w.hbi, w.hal, s * w.hbl, w.har, s * w.hbr);
 }
 
+// Potential stage of one cell: p psi (INVERSE: at the stage's output, else at
+// its input), l lambda at its output; e the table's entry, g dL/dV of the cell.
+// IMAGINARY: kf sd is the cell's part of Re<Lambda_k, psi_k>.
+template <class A>
+__device__ __forceinline__ void adj_cell(const AdjArgs &a, Cx<double> &p, Cx<double> &l,
+                                         typename A::TabT e, double &g, double &kf, double &sd) {
+    const double n2 = __fma_rn(p.re, p.re, __dmul_rn(p.im, p.im));
+    double th = 0.0, dth = 0.0;
+    if (A::PHASE) {
+        th = __dmul_rn(a.ca, n2);
+        dth = a.ca;
+        if (A::PHASE == 2) {
+            const double r = sqrt(n2);
+            th = __fma_rn(a.caa, __dmul_rn(n2, r), th);
+            dth = __fma_rn(1.5 * a.caa, r, dth);
+        }
+    }
+    if constexpr (A::IMAG) {
+        const double fe = A::PHASE ? __dmul_rn(phase_expneg(th), e) : e;
+        sd = __fma_rn(l.re, p.re, __dmul_rn(l.im, p.im));
+        const double k2 = 2.0 * dth * sd;
+        g = __fma_rn(-a.dt, __dmul_rn(fe, sd), g);
+        kf = __dmul_rn(fe, __fma_rn(-2.0 * dth, n2, 1.0));
+        l.re = __dmul_rn(fe, __fma_rn(-k2, p.re, l.re));
+        l.im = __dmul_rn(fe, __fma_rn(-k2, p.im, l.im));
+    } else if constexpr (A::MODE == 0) {
+        const double qv = __fma_rn(l.re, p.im, -__dmul_rn(l.im, p.re));
+        g = __fma_rn(a.dt, qv, g);
+        p = Cx<double>{__fma_rn(e.re, p.re, __dmul_rn(e.im, p.im)),
+                       __fma_rn(e.re, p.im, -__dmul_rn(e.im, p.re))};
+        l = Cx<double>{__fma_rn(e.re, l.re, __dmul_rn(e.im, l.im)),
+                       __fma_rn(e.re, l.im, -__dmul_rn(e.im, l.re))};
+    } else {
+        double c = 1.0, s = 0.0;
+        if (A::PHASE) phase_sincos(th, &s, &c);
+        // psi' = exp(-i theta) (E x)
+        const double tr = __fma_rn(e.re, p.re, -__dmul_rn(e.im, p.im));
+        const double ti = __fma_rn(e.re, p.im, __dmul_rn(e.im, p.re));
+        const double pr = __fma_rn(c, tr, __dmul_rn(s, ti));
+        const double pi = __fma_rn(c, ti, -__dmul_rn(s, tr));
+        const double qv = __fma_rn(l.re, pi, -__dmul_rn(l.im, pr));
+        g = __fma_rn(a.dt, qv, g);
+        // lambda = conj(E) exp(+i theta) lambda' + 2 theta' q x
+        const double ur = __fma_rn(c, l.re, -__dmul_rn(s, l.im));
+        const double ui = __fma_rn(c, l.im, __dmul_rn(s, l.re));
+        const double k2 = A::PHASE ? 2.0 * dth * qv : 0.0;
+        l.re = __fma_rn(e.re, ur, __fma_rn(e.im, ui, __dmul_rn(k2, p.re)));
+        l.im = __fma_rn(e.re, ui, __fma_rn(-e.im, ur, __dmul_rn(k2, p.im)));
+    }
+}
+
 // Potential stage of row u (both fields at this point of the pipeline).
 template <class A>
 __device__ __forceinline__ void adj_potential(AdjWalk &w, const AdjArgs &a, Cx<double> (&ps)[2],
                                               Cx<double> (&la)[2], int q, int u) {
     const unsigned char *sb = w.ring + q * A::SLOT;
     const double *gp = reinterpret_cast<const double *>(sb + A::GV_OFF) + 2 * w.lane;
+    const typename A::TabT *ep =
+        reinterpret_cast<const typename A::TabT *>(sb + A::TAB_OFF) + 2 * w.lane;
     const bool out_row = u >= w.oy0 && u < w.oy1;
     double *grow = a.gv + (size_t)u * a.P + w.xl;
-    if constexpr (A::IMAG) {
-        const double *ep = reinterpret_cast<const double *>(sb + A::TAB_OFF) + 2 * w.lane;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            // psi is chi (the stage's input), lambda is at the stage's output
-            const Cx<double> x = ps[i];
-            const Cx<double> l = la[i];
-            const double n2 = __fma_rn(x.re, x.re, __dmul_rn(x.im, x.im));
-            double th = 0.0, dth = 0.0;
-            if (A::PHASE) {
-                th = __dmul_rn(a.ca, n2);
-                dth = a.ca;
-                if (A::PHASE == 2) {
-                    const double r = sqrt(n2);
-                    th = __fma_rn(a.caa, __dmul_rn(n2, r), th);
-                    dth = __fma_rn(1.5 * a.caa, r, dth);
-                }
-            }
-            const double fe = A::PHASE ? __dmul_rn(phase_expneg(th), ep[i]) : ep[i];
-            const double sd = __fma_rn(l.re, x.re, __dmul_rn(l.im, x.im));
-            const double k2 = 2.0 * dth * sd;
-            if (out_row && w.out_col[i]) {
-                grow[i] = __fma_rn(-a.dt, __dmul_rn(fe, sd), gp[i]);
-                w.kacc = __fma_rn(__dmul_rn(fe, __fma_rn(-2.0 * dth, n2, 1.0)), sd, w.kacc);
-            }
-            la[i].re = __dmul_rn(fe, __fma_rn(-k2, x.re, l.re));
-            la[i].im = __dmul_rn(fe, __fma_rn(-k2, x.im, l.im));
-        }
-        return;
-    }
-    const Cx<double> *tp = reinterpret_cast<const Cx<double> *>(sb + A::TAB_OFF) + 2 * w.lane;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const Cx<double> e = ld_cx_shared(tp + i);
-        const double g_old = gp[i];
-        const Cx<double> l = la[i];
-        if (A::MODE == 0) {
-            // psi, lambda are at the stage's output: psi' and lambda'
-            const Cx<double> p = ps[i];
-            const double qv = __fma_rn(l.re, p.im, -__dmul_rn(l.im, p.re));
-            if (out_row && w.out_col[i]) grow[i] = __fma_rn(a.dt, qv, g_old);
-            ps[i].re = __fma_rn(e.re, p.re, __dmul_rn(e.im, p.im));
-            ps[i].im = __fma_rn(e.re, p.im, -__dmul_rn(e.im, p.re));
-            la[i].re = __fma_rn(e.re, l.re, __dmul_rn(e.im, l.im));
-            la[i].im = __fma_rn(e.re, l.im, -__dmul_rn(e.im, l.re));
-        } else {
-            // psi is at the stage's input, lambda at its output
-            const Cx<double> x = ps[i];
-            const double n2 = __fma_rn(x.re, x.re, __dmul_rn(x.im, x.im));
-            double c = 1.0, s = 0.0, dth = 0.0;
-            if (A::PHASE) {
-                double th = __dmul_rn(a.ca, n2);
-                dth = a.ca;
-                if (A::PHASE == 2) {
-                    const double r = sqrt(n2);
-                    th = __fma_rn(a.caa, __dmul_rn(n2, r), th);
-                    dth = __fma_rn(1.5 * a.caa, r, dth);
-                }
-                phase_sincos(th, &s, &c);
-            }
-            // psi' = exp(-i theta) (E x)
-            const double tr = __fma_rn(e.re, x.re, -__dmul_rn(e.im, x.im));
-            const double ti = __fma_rn(e.re, x.im, __dmul_rn(e.im, x.re));
-            const double pr = __fma_rn(c, tr, __dmul_rn(s, ti));
-            const double pi = __fma_rn(c, ti, -__dmul_rn(s, tr));
-            const double qv = __fma_rn(l.re, pi, -__dmul_rn(l.im, pr));
-            if (out_row && w.out_col[i]) grow[i] = __fma_rn(a.dt, qv, g_old);
-            // lambda = conj(E) exp(+i theta) lambda' + 2 theta' q x
-            const double ur = __fma_rn(c, l.re, -__dmul_rn(s, l.im));
-            const double ui = __fma_rn(c, l.im, __dmul_rn(s, l.re));
-            const double k2 = A::PHASE ? 2.0 * dth * qv : 0.0;
-            la[i].re = __fma_rn(e.re, ur, __fma_rn(e.im, ui, __dmul_rn(k2, x.re)));
-            la[i].im = __fma_rn(e.re, ui, __fma_rn(-e.im, ur, __dmul_rn(k2, x.im)));
+        double g = gp[i], kf = 0.0, sd = 0.0;
+        typename A::TabT e;
+        if constexpr (A::IMAG) e = ep[i];
+        else e = ld_cx_shared(ep + i);
+        adj_cell<A>(a, ps[i], la[i], e, g, kf, sd);
+        if (out_row && w.out_col[i]) {
+            grow[i] = g;
+            if constexpr (A::IMAG) w.kacc = __fma_rn(kf, sd, w.kacc);
         }
     }
 }
@@ -352,6 +343,39 @@ __device__ __forceinline__ void adj_rows(AdjWalk &w, const AdjArgs &a, int base,
         if (w.failed || (GUARD && r > rlast)) return;
         adj_row<A, K, GUARD>(w, a, r);
         adj_rows<A, K + 1, GUARD>(w, a, base, rlast);
+    }
+}
+
+// IMAGINARY: Re<Lambda_k, psi_k> from the lanes' parts: warps of the block, then
+// the blocks in a fixed order by the last block to finish.
+__device__ __forceinline__ void adj_finish(const AdjArgs &a, double v, int warps, int warp,
+                                           int lane) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    __shared__ double s_warp[32];
+    __shared__ unsigned int s_last;
+    if (lane == 0) s_warp[warp] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double b = 0.0;
+        for (int i = 0; i < warps; ++i) b += s_warp[i];
+        a.partials[blockIdx.x] = b;
+        __threadfence();
+        s_last = (atomicAdd(a.ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
+    }
+    __syncthreads();
+    if (s_last && warp == 0) {
+        // all loads in flight, then the lanes' sums in order
+        __threadfence();
+        double t = 0.0;
+        for (int i = lane; i < (int)gridDim.x; i += 32) t += __ldcg(&a.partials[i]);
+        double tot = 0.0;
+        for (int i = 0; i < 32; ++i) tot += __shfl_sync(0xffffffffu, t, i);
+        if (lane == 0) {
+            *a.mu_out = a.mu_scale * tot;
+            if (a.accumulate) *a.kappa_sum += tot;
+            *a.ticket = 0u;
+        }
     }
 }
 
@@ -488,33 +512,7 @@ __global__ void __launch_bounds__(64, 6) adjoint_kernel(AdjArgs a) {
             }
         }
     }
-    if constexpr (A::IMAG) {
-        // Re<Lambda_k, psi_k>: lanes, warps of the block, then the blocks in
-        // a fixed order by the last block to finish
-        double v = w.kacc;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        __shared__ double s_warp[32];
-        __shared__ unsigned int s_last;
-        if (lane == 0) s_warp[warp] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double b = 0.0;
-            for (int i = 0; i < warps; ++i) b += s_warp[i];
-            a.partials[blockIdx.x] = b;
-            __threadfence();
-            s_last = (atomicAdd(a.ticket, 1u) == gridDim.x - 1) ? 1u : 0u;
-        }
-        __syncthreads();
-        if (s_last && threadIdx.x == 0) {
-            __threadfence();
-            double tot = 0.0;
-            for (int i = 0; i < (int)gridDim.x; ++i) tot += __ldcg(&a.partials[i]);
-            *a.mu_out = a.mu_scale * tot;
-            if (a.accumulate) *a.kappa_sum += tot;
-            *a.ticket = 0u;
-        }
-    }
+    if constexpr (A::IMAG) adj_finish(a, w.kacc, warps, warp, lane);
 }
 
 }  // namespace tsb

@@ -70,6 +70,28 @@ struct Patch {
     unsigned hm, vm;      // EDGE: bit i + 1: the pair (i, i + 1) crosses the tile's edge
 };
 
+// This thread's place in the region; exch: the block's exchange buffers.
+template <class S>
+__device__ __forceinline__ void patch_thread(Patch<S> &p, unsigned char *exch) {
+    using T = typename S::T;
+    const int lane = threadIdx.x & 31;
+    p.px = (int)(threadIdx.x >> 5) * S::WX + lane % S::WX;
+    p.py = lane / S::WX;
+    p.exch = exch + threadIdx.x * (int)sizeof(Cx<T>);
+    // the outer edge's neighbour is the other column of the next warp
+    p.outer = (p.px == 0 || p.px == S::TX - 1) ? 0
+                                               : (p.px & 1 ? 31 : -31) * (int)sizeof(Cx<T>);
+    p.hm = p.vm = 0u;
+}
+
+// EDGE: the pairs of this patch that cross the edge of a W x H tile.
+template <class S>
+__device__ __forceinline__ void patch_masks(Patch<S> &p, int W, int H) {
+    const int rx = W - p.gx, ry = H - p.gy;  // cells to the tile's end
+    p.hm = (p.gx == 0 ? 1u : 0u) | ((rx >= 0 && rx <= S::N) ? 1u << rx : 0u);
+    p.vm = (p.gy == 0 ? 1u : 0u) | ((ry >= 0 && ry <= S::N) ? 1u << ry : 0u);
+}
+
 template <class T>
 __device__ __forceinline__ T patch_one() {
     return DeltaForm<T>::value ? T(0) : T(1);
@@ -353,12 +375,15 @@ struct PatchTile {
     int P;
     bool whole;       // EDGE: no cell of a row outside the tile or wrapped in x
 
-    __device__ __forceinline__ PatchTile(const Patch<S> &p, const StepArgs<T> &a, const void *tile)
+    template <class Args>
+    __device__ __forceinline__ PatchTile(const Patch<S> &p, const Args &a, const void *tile)
         : at(reinterpret_cast<const Cx<T> *>(tile) + (ptrdiff_t)p.gy * a.P + p.gx), P(a.P) {
-        const int wx = (WRAP && (a.wrap & 1)) ? a.wrap_hx : 0;
+        int wx = 0;
+        if constexpr (WRAP) wx = (a.wrap & 1) ? a.wrap_hx : 0;
         whole = !EDGE || (p.gx >= wx && p.gx + N <= a.W - wx);
     }
-    __device__ __forceinline__ void row(const Patch<S> &p, const StepArgs<T> &a, int j,
+    template <class Args>
+    __device__ __forceinline__ void row(const Patch<S> &p, const Args &a, int j,
                                         Cx<T> (&v)[N]) const {
         alignas(16) Cx<T> w[N];
         if constexpr (!EDGE) {
@@ -369,22 +394,27 @@ struct PatchTile {
             const int y = p.gy + j;
             if (y >= 0 && y < a.H) {
                 int dy = j;
-                if (WRAP && (a.wrap & 2)) {
-                    if (y < a.wrap_hy) dy += a.H - 2 * a.wrap_hy;
-                    else if (y >= a.H - a.wrap_hy) dy -= a.H - 2 * a.wrap_hy;
+                if constexpr (WRAP) {
+                    if (a.wrap & 2) {
+                        if (y < a.wrap_hy) dy += a.H - 2 * a.wrap_hy;
+                        else if (y >= a.H - a.wrap_hy) dy -= a.H - 2 * a.wrap_hy;
+                    }
                 }
                 const Cx<T> *r = at + (ptrdiff_t)dy * P;
                 if (whole) {
                     patch_ld<N * (int)sizeof(Cx<T>)>(r, w);
                 } else {
-                    const int ys = p.gy + dy, n_in = a.W - 2 * a.wrap_hx;
-                    const bool wrap = WRAP && (a.wrap & 1) && ys >= a.wrap_y0 && ys < a.wrap_y1;
+                    const int ys = p.gy + dy;
 #pragma unroll
                     for (int i = 0; i < N; ++i) {
                         const int x = p.gx + i;
                         int dx = i;
-                        if (wrap && x < a.wrap_hx) dx += n_in;
-                        else if (wrap && x >= a.W - a.wrap_hx) dx -= n_in;
+                        if constexpr (WRAP) {
+                            if ((a.wrap & 1) && ys >= a.wrap_y0 && ys < a.wrap_y1) {
+                                if (x < a.wrap_hx) dx += a.W - 2 * a.wrap_hx;
+                                else if (x >= a.W - a.wrap_hx) dx -= a.W - 2 * a.wrap_hx;
+                            }
+                        }
                         if (x >= 0 && x < a.W) w[i] = ld_cx_shared(r + dx);
                     }
                 }
@@ -406,12 +436,15 @@ struct PatchTable {
     ptrdiff_t pitch;
     bool whole;
 
-    __device__ __forceinline__ PatchTable(const Patch<S> &p, const StepArgs<T> &a) {
-        pitch = S::V::VPOT ? (ptrdiff_t)(a.pot_pitch / sizeof(TabT)) : (ptrdiff_t)a.P;
+    template <class Args>
+    __device__ __forceinline__ PatchTable(const Patch<S> &p, const Args &a) {
+        pitch = a.P;
+        if constexpr (S::V::VPOT) pitch = (ptrdiff_t)(a.pot_pitch / sizeof(TabT));
         at = reinterpret_cast<const TabT *>(a.pot) + p.gy * pitch + p.gx;
         whole = !EDGE || (p.gx >= 0 && p.gx + N <= a.W);
     }
-    __device__ __forceinline__ void row(const Patch<S> &p, const StepArgs<T> &a, int j,
+    template <class Args>
+    __device__ __forceinline__ void row(const Patch<S> &p, const Args &a, int j,
                                         TabT (&v)[N]) const {
         alignas(16) TabT w[N];
 #pragma unroll
@@ -480,11 +513,7 @@ __device__ __forceinline__ void patch_region(Patch<S> &p, const StepArgs<typenam
     constexpr bool WRAP = !V::PB;
     p.gx = X0 + p.px * N;
     p.gy = Y0 + p.py * N;
-    if constexpr (EDGE) {
-        const int rx = a.W - p.gx, ry = a.H - p.gy;  // cells to the tile's end
-        p.hm = (p.gx == 0 ? 1u : 0u) | ((rx >= 0 && rx <= N) ? 1u << rx : 0u);
-        p.vm = (p.gy == 0 ? 1u : 0u) | ((ry >= 0 && ry <= N) ? 1u << ry : 0u);
-    }
+    if constexpr (EDGE) patch_masks(p, a.W, a.H);
     const PatchTile<S, EDGE, WRAP> tile(p, a, a.psi_in);
     const PatchTable<S, EDGE> table(p, a);
 #pragma unroll
@@ -600,13 +629,7 @@ __global__ void __launch_bounds__(S::THREADS, S::BLOCKS) patch_kernel(StepArgs<t
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     Patch<S> p;
-    p.px = warp * S::WX + lane % S::WX;
-    p.py = lane / S::WX;
-    p.exch = exch + threadIdx.x * (int)sizeof(Cx<T>);
-    // the outer edge's neighbour is the other column of the next warp
-    p.outer = (p.px == 0 || p.px == S::TX - 1) ? 0
-                                               : (p.px & 1 ? 31 : -31) * (int)sizeof(Cx<T>);
-    p.hm = p.vm = 0u;
+    patch_thread(p, exch);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     p.aH = a.aH;
     p.bH = a.bH;
