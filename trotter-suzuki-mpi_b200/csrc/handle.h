@@ -18,15 +18,16 @@ struct ts_b200_kernel {
     int phase = 0;  // 0 none, 1 g|psi|^2, 2 with Lee-Huang-Yang, 3 one component of a pair
                     // (7: the same with the Rabi rotation applied at load), | 4 cylindrical
     size_t cell = 0, tab_cell = 0;
+    void *memory = nullptr;  // all buffers below but own_partials and own_vtab
     void *psi[2] = {nullptr, nullptr};
     int cur = 0;
     void *tab = nullptr;
     void *row_ab = nullptr, *col_ab = nullptr;
-    double *partials = nullptr;
+    double *partials = nullptr, *own_partials = nullptr;
     size_t partials_cap = 0;
     tsb::Scalars *scal = nullptr;
     double *staging = nullptr;  // 2 * W * H doubles
-    double *vtab = nullptr;     // V for energies (W * H)
+    double *vtab = nullptr, *own_vtab = nullptr;  // V for energies (W * H)
     bool have_v = false;
     double *red_partials = nullptr;
     double *red_out = nullptr;
