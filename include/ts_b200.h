@@ -118,7 +118,9 @@ int ts_b200_halo_exchange(ts_b200_kernel *k);
 
 /* `iterations` steps with the reference's evolve() semantics: the halo is
  * refreshed after every step but the last (src/solver.cpp:186-230).  Steps
- * are replayed from a CUDA graph; nothing synchronises the host. */
+ * are replayed from a CUDA graph; nothing synchronises the host.  Small and
+ * middle-sized closed tiles in real time take 2 or 3 steps per launch, unless a
+ * walk or its shape has been asked for. */
 int ts_b200_evolve(ts_b200_kernel *k, int iterations);
 
 /* Copy a width x height window at (x, y) of the tile to host SoA arrays with

@@ -177,6 +177,36 @@ def test_patches_with_potential_rows(W, H, pad):
     assert np.array_equal(out[None], out[0])
 
 
+# sizes with 8 or 16 written cells per region (3 or 2 steps of 2 x 2 patches), on
+# either side of the limit between them, and with 48 (2 steps of 4 x 4)
+@pytest.mark.parametrize("N,Ny,precision", [
+    (1, 1, 0), (8, 8, 0), (9, 17, 1), (41, 30, 0), (97, 97, 0), (112, 113, 1), (256, 255, 0),
+    (301, 304, 0), (391, 390, 1), (501, 530, 0), (770, 815, 0), (1150, 1201, 1)])
+@pytest.mark.parametrize("g,lhy", [(0.0, 0.0), (2.0, 0.0), (2.0, 0.3)])
+def test_several_steps_per_launch_match_single_steps(N, Ny, precision, g, lhy):
+    """evolve() of odd and even numbers of steps, from either buffer, plain and
+    replayed: the bits of as many single steps."""
+    from trottersuzuki_b200 import Kernel
+    lat, psi0, V = seeded_case(N, 0.05 * N, Ny)
+    desc = desc_from_params(lat.params(1e-3, False, 1.0, g, lhy), precision=precision)
+    pot = np.exp(-1e-3j * V)
+    out = []
+    for single in (False, True):
+        k = Kernel(desc)
+        k.set_state(psi0)
+        k.set_exp_potential(pot.real.copy(), pot.imag.copy())
+        for n in (1, 2, 3, 4, 5, 50, 99):
+            if single:
+                for _ in range(n):
+                    k.step(exchange=False)
+            else:
+                k.evolve(n)
+        out.append(k.get_state())
+        k.close()
+    assert np.isfinite(out[0]).all()
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("N,Ny", [(1, 1), (24, 24), (25, 49), (131, 90)])
 @pytest.mark.parametrize("g,lhy,every,imag", [(0.0, 0.0, 0, False), (8.0, 0.0, 4, False),
                                               (8.0, 0.5, 3, False), (0.0, 0.0, 5, True),

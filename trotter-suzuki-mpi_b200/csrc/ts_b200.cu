@@ -928,8 +928,6 @@ int configure_t(ts_b200_kernel *k) {
     return TS_B200_OK;
 }
 
-// One fused step from buffer `in` to buffer `out` (no buffer flip, no halo);
-// dry: configure and size the scratch only.
 // Block sums of an imaginary-time step beyond those of the handle's allocation.
 int grow_partials(ts_b200_kernel *k, size_t n) {
     if (k->own_partials) cudaFree(k->own_partials);
@@ -941,6 +939,8 @@ int grow_partials(ts_b200_kernel *k, size_t n) {
     return TS_B200_OK;
 }
 
+// One fused step from buffer `in` to buffer `out` (no buffer flip, no halo);
+// dry: configure and size the scratch only.
 template <typename T>
 int launch_step_buffers_t(ts_b200_kernel *k, const void *in, void *out, bool dry) {
     int strips, segs, blocks;
@@ -994,6 +994,82 @@ int launch_step_t(ts_b200_kernel *k, int exchange, bool dry = false) {
     }
     k->wrap_next = exchange && k->wrap_steps;
     return TS_B200_OK;
+}
+
+// Steps of one launch inside ts_b200_evolve (patch_region_steps) and cells per
+// side of a thread's patch; m = 1 where steps are launched one by one: what is
+// not a closed tile in plain real time, and where a walk or its shape has been
+// asked for.  Three steps of 32 x 32 regions while each has an SM of its own, two
+// while they are resident at once (a quarter more in double), two of 64 x 64
+// regions where these fill the SMs.  us per step on square tiles, 3 steps of 2 x 2
+// patches / 2 steps / 2 steps of 4 x 4 / launched one by one:
+//   double, GPE: 64^2 1.81 / 1.91 / - / 3.13, 128^2 2.28 / 2.20 / - / 3.40, 256^2 -
+//     / 2.55 / - / 3.60, 300^2 - / 3.68 / 5.95 / 4.24, 384^2 - / 4.52 / 6.05 /
+//     4.43, 480^2 - / - / 6.11 / 4.91, 576^2 - / - / 6.31 / 7.42, 816^2 - / - /
+//     8.74 / 11.81, 900^2 - / - / 13.5 / 13.5
+//   linear: 64^2 1.55 / 1.71 / - / 2.88, 512^2 - / - / 5.28 / 5.98; with
+//     Lee-Huang-Yang 300^2 - / 4.77 / 8.46 / 4.94, 640^2 - / - / 10.7 / 9.5, 720^2
+//     - / - / 11.3 / 11.9, 816^2 - / - / 11.5 / 13.4
+//   float, GPE: 64^2 1.98 / 2.49 / - / 4.31, 256^2 - / 3.31 / - / 5.09, 384^2 - /
+//     4.16 / 5.03 / 5.61, 512^2 - / 6.81 / 4.97 / 6.54, 816^2 - / - / 6.45 / 9.79,
+//     1200^2 - / - / 12.8 / 14.1, 1400^2 - / - / 16.5 / 15.8; with Lee-Huang-Yang
+//     512^2 - / - / 7.62 / 7.12, 816^2 - / - / 8.2 / 11.1, 1200^2 16.8 / 18.1
+struct Fused {
+    int n = 0, m = 1;
+    int nx = 0, ny = 0;  // regions
+};
+
+Fused fused_steps(const ts_b200_kernel *k) {
+    Fused f;
+    if (!k->patch || k->walk2 != 2 || k->imag || k->rot || k->phase > 2 || k->pair_mode ||
+        k->vpot || k->d.periodic_x || k->d.periodic_y)
+        return f;
+    const int sms = k->num_sms;
+    const bool lhy = k->phase == 2;
+    auto take = [&](int n, int m, int more_than, int most) {
+        const int out = tsb::patch_out(n, 4 * m);
+        const long nx = div_up(k->W, out), ny = div_up(k->H, out);
+        if (nx * ny <= more_than || nx * ny > most) return false;
+        f = Fused{n, m, (int)nx, (int)ny};
+        return true;
+    };
+    if (take(2, 3, 0, sms)) return f;
+    if (take(2, 2, 0, k->fp32 ? 4 * sms : 5 * sms / 2)) return f;
+    if (k->fp32)
+        take(4, 2, lhy ? 5 * sms / 4 : 0, 17 * sms / 4);
+    else
+        take(4, 2, lhy ? 7 * sms / 5 : 3 * sms / 4, 2 * sms);
+    return f;
+}
+
+// f.m steps from buffer `in` to buffer `out` (no buffer flip).
+template <typename T>
+int launch_fused_buffers_t(ts_b200_kernel *k, const Fused &f, const void *in, void *out) {
+    StepArgs<T> a{};
+    a.psi_in = in;
+    a.psi_out = out;
+    tsbh::fill_step_constants(k, a);
+    a.n_strips = f.nx;
+    a.n_segs = f.ny;
+    const int most = tsb::patch_steps_blocks(f.n, k->fp32) * k->num_sms;
+    const int blocks = std::min(f.nx * f.ny, most);
+    // as step_pdl: not where the next launch's blocks would crowd some of the SMs
+    // (us per step without / with, double GPE: 96^2 in 144 blocks of at most 296
+    // 1.73 / 2.13, 256^2 in 256 2.89 / 2.55; 4 x 4 patches 512^2 in 121 6.2 / 7.9,
+    // 720^2 in 225 8.6 / 8.4; float 256^2 in 256 of 592 3.3 / 3.9)
+    const bool pdl = k->overlap_set ? walk_pdl(k)
+                                    : 2 * blocks <= k->num_sms ||
+                                          (f.n == 4 ? blocks > k->num_sms
+                                                    : 20 * blocks >= 17 * most);
+    const cudaError_t e = tsb::launch_patch_steps(f.n, f.m, k->phase, a, blocks, k->stream, pdl);
+    if (e != cudaSuccess) return cuda_fail(k, e, "fused steps launch");
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TS_B200_OK;
+}
+
+int launch_fused_buffers(ts_b200_kernel *k, const Fused &f, const void *in, void *out) {
+    return k->fp32 ? launch_fused_buffers_t<float>(k, f, in, out)
+                   : launch_fused_buffers_t<double>(k, f, in, out);
 }
 
 int launch_step(ts_b200_kernel *k, int exchange, bool dry = false) {
@@ -1658,9 +1734,10 @@ int ts_b200_evolve(ts_b200_kernel *k, int iterations) {
     if (iterations == 0) return TS_B200_OK;
     // Steps 0 .. iterations-2 refresh the halo; the last one does not
     // (src/solver.cpp:203-209).  Runs of G exchanging steps starting from
-    // buffer 0 are replayed from one CUDA graph (G even, so the graph leaves
-    // the buffers as it found them).
-    const int G = 32;
+    // buffer 0 are replayed from one CUDA graph (an even number of launches,
+    // so the graph leaves the buffers as it found them).
+    const Fused fused = fused_steps(k);
+    const int G = 16 * std::max(fused.m, 2);
     int remaining = iterations - 1;  // exchanging steps
     // The patch step reads the halo of the previous step's output from the
     // cells the refresh would copy (no refresh launch): every step but the
@@ -1670,14 +1747,21 @@ int ts_b200_evolve(ts_b200_kernel *k, int iterations) {
         ts_b200_kernel *k;
         ~Reset() { k->wrap_steps = k->wrap_next = false; }
     } reset{k};
-    // plain steps up to buffer 0 and, with wrapped steps, past the first one
-    // (the graph's first step wraps)
-    while (remaining > 0 && (k->cur != 0 || (k->wrap_steps && !k->wrap_next))) {
+    // one launch of f.m steps (of one exchanging step)
+    auto launch = [k](const Fused &f) {
+        if (f.m == 1) return launch_step(k, 1);
+        const int s = launch_fused_buffers(k, f, k->psi[k->cur], k->psi[1 - k->cur]);
+        if (s == TS_B200_OK) k->cur = 1 - k->cur;
+        return s;
+    };
+    // plain steps up to buffer 0 for the graph and, with wrapped steps, past the
+    // first one (the graph's first step wraps)
+    while (remaining > 0 && ((k->cur != 0 && remaining > G) || (k->wrap_steps && !k->wrap_next))) {
         int s = launch_step(k, 1);
         if (s) return s;
         --remaining;
     }
-    if (remaining >= G) {
+    if (remaining >= G && k->cur == 0) {
         if (!k->graph || k->graph_steps != G) {
             drop_graph(k);
             int s0 = launch_step(k, 1, true);  // scratch and attributes before capture
@@ -1686,7 +1770,7 @@ int ts_b200_evolve(ts_b200_kernel *k, int iterations) {
             TSB_CHECK(k, cudaStreamBeginCapture(k->stream, cudaStreamCaptureModeThreadLocal));
             const uint64_t before = g_launches.load();
             int s = TS_B200_OK;
-            for (int i = 0; i < G && s == TS_B200_OK; ++i) s = launch_step(k, 1);
+            for (int i = 0; i < G && s == TS_B200_OK; i += fused.m) s = launch(fused);
             cudaError_t e = cudaStreamEndCapture(k->stream, &g);
             g_launches.store(before);  // captured launches are counted when replayed
             if (s != TS_B200_OK || e != cudaSuccess) {
@@ -1700,18 +1784,25 @@ int ts_b200_evolve(ts_b200_kernel *k, int iterations) {
             if (e != cudaSuccess) return cuda_fail(k, e, "graph instantiate");
             k->graph_steps = G;
         }
-        const int per = kernels_per_step(k, 1);
+        const int launches = G / fused.m * kernels_per_step(k, 1);
         while (remaining >= G) {
             TSB_CHECK(k, cudaGraphLaunch(k->graph, k->stream));
-            g_launches.fetch_add((uint64_t)G * per, std::memory_order_relaxed);
+            g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
             remaining -= G;
         }
     }
-    for (; remaining > 0; --remaining) {
-        int s = launch_step(k, 1);
+    // a closed tile's last step is a step like the others
+    if (fused.m > 1) ++remaining;
+    for (; remaining >= fused.m; remaining -= fused.m) {
+        int s = launch(fused);
         if (s) return s;
     }
-    return launch_step(k, 0);
+    if (fused.m == 1) return launch_step(k, 0);
+    for (; remaining > 0; --remaining) {
+        int s = launch_step(k, 0);
+        if (s) return s;
+    }
+    return TS_B200_OK;
 }
 
 int ts_b200_get_sample(ts_b200_kernel *k, size_t dest_stride, size_t x, size_t y, size_t width,
@@ -1950,19 +2041,26 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
     int st = TS_B200_OK;
     // trial_steps steps of the current choice, after one untimed
     auto time_steps = [&](float *ms) {
-        int s = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
+        const Fused f = fused_steps(k);
+        auto launch = [&] {
+            const void *in = k->psi[k->cur];
+            void *out = k->psi[1 - k->cur];
+            return f.m > 1 ? launch_fused_buffers(k, f, in, out)
+                           : tsbh::launch_step_buffers(k, in, out);
+        };
+        int s = launch();
         if (s) return s;
         cudaEventRecord(e0, k->stream);
-        for (int i = 0; i < trial_steps && s == TS_B200_OK; ++i)
-            s = tsbh::launch_step_buffers(k, k->psi[k->cur], k->psi[1 - k->cur]);
+        for (int i = 0; i < trial_steps && s == TS_B200_OK; ++i) s = launch();
         cudaEventRecord(e1, k->stream);
         cudaError_t e = cudaEventSynchronize(e1);
         if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
+        *ms /= (float)f.m;
         if (s == TS_B200_OK && e != cudaSuccess) s = cuda_fail(k, e, "autotune timing");
         return s;
     };
     // the register patches, where they are this tile's default
-    if (patch_cells(k)) {
+    if (patch_cells(k) || fused_steps(k).m > 1) {
         st = time_steps(&best_ms);
         best_patch = st == TS_B200_OK;
     }

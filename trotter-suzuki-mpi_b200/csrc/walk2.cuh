@@ -762,7 +762,8 @@ __device__ __forceinline__ void w2_task(Walk2<V, R> &w, const StepArgs<typename 
 constexpr int kFinishScratch = 65;
 template <class V>
 __device__ __forceinline__ void w2_finish(const StepArgs<typename V::T> &a, double nacc, int warps,
-                                          int warp, int lane, double *scratch) {
+                                          int warp, int lane, double *scratch,
+                                          unsigned int steps = 1u) {
     if constexpr (!V::IMAG && DeltaForm<typename V::T>::value) {
         if (a.kin_sched) {
             __syncthreads();
@@ -771,7 +772,7 @@ __device__ __forceinline__ void w2_finish(const StepArgs<typename V::T> &a, doub
                 unsigned int *tk = launch_ticket(a);
                 if (atomicAdd(tk, 1u) == gridDim.x - 1) {
                     *tk = 0u;
-                    if (step_ends_here(a)) a.scal->step += 1u;
+                    if (step_ends_here(a)) a.scal->step += steps;
                     __threadfence();
                 }
             }
