@@ -390,7 +390,8 @@ int ts_b200_batch_synchronize(ts_b200_batch *b);
 int ts_b200_batch_set_stream(ts_b200_batch *b, void *stream);
 
 /* Tile shape of the batched launch: rows per segment task (even; capped by
- * each tile's height) and warps per block (1, 2 or 4).  Zero keeps a field. */
+ * each tile's height) and warps per block (1, 2 or 4).  Zero keeps a field; until
+ * rows are asked for or autotuned they are chosen by the tiles' sizes. */
 int ts_b200_batch_set_launch(ts_b200_batch *b, int segment_rows, int warps_per_block);
 
 /* Autotuner: times `trial_steps` batched steps for each candidate shape (rows

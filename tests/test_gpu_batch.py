@@ -222,3 +222,23 @@ def test_solver_batch_matches_solver_loop(imag):
             assert np.array_equal(a, b)
             assert s1.get_total_energy() == s2.get_total_energy()
     sb.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("sizes", [[(5, 3), (56, 8), (57, 9)], [(300, 290)] * 6,
+                                   [(3000, 3000), (2700, 2990), (61, 47)]],
+                         ids=["shortest", "one_task_per_warp", "several_per_warp"])
+def test_default_segments_are_bitwise_per_tile(sizes, precision):
+    """The rows per segment that the batch chooses: the shortest, one task per
+    warp, and tasks taken in turns."""
+    from trottersuzuki_b200 import Batch
+    tiles = make_tiles(False, precision, tiles=[
+        (f"{n}x{ny}", n, 0.2 * n, ny, (False, False), 2.0, 0.0) for n, ny in sizes])
+    with Batch([t["k"] for t in tiles]) as b:
+        b.evolve(3)
+        b.synchronize()
+        got = [t["k"].get_state() for t in tiles]
+    ref = individual(tiles, [3], precision)
+    close_all(tiles)
+    for t, g, r in zip(tiles, got, ref):
+        assert np.array_equal(g, r), f"{t['name']}: max|d| = {np.abs(g - r).max():.3e}"

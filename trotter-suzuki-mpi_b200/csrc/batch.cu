@@ -104,6 +104,7 @@ struct ts_b200_batch {
     int phase = 0;
     int device = 0, num_sms = 148;
     Shape shape{128, 4};
+    bool auto_seg = true;  // choose the rows per segment (auto_segment)
     // row walk: 2 the look-ahead walk (two rows per iteration, a ring of 6
     // rows), 0 the checked walk (a ring of `ring` rows)
     int walk = 0;
@@ -163,14 +164,64 @@ int batch_vlen(const ts_b200_batch *b) {
     return tsb::w2_vlen(seg, false);
 }
 
-size_t batch_smem(const ts_b200_batch *b, int warps) {
+size_t batch_smem(const ts_b200_batch *b, int warps, int vlen) {
     if (b->walk) {
         // per warp: the ring, the vertical pair table and one mbarrier per
         // ring slot of two rows
         return (size_t)warps * (b->ring * tsbh::slot_bytes(2, b->fp32, b->imag) +
-                                (size_t)batch_vlen(b) * (b->fp32 ? 8 : 16) + (b->ring / 2) * 8);
+                                (size_t)vlen * (b->fp32 ? 8 : 16) + (b->ring / 2) * 8);
     }
     return (size_t)warps * (b->ring * tsbh::slot_bytes(2, b->fp32, b->imag) + 8 * b->ring);
+}
+size_t batch_smem(const ts_b200_batch *b, int warps) {
+    return batch_smem(b, warps, batch_vlen(b));
+}
+
+// Rows per segment: one task per warp with 4, 8, 12 or 16 warps per SM, as for
+// a single tile (auto_segments in ts_b200.cu): the walked rows, with the
+// segment's 8 halo rows, times what a row costs at that many warps are
+// fewest.  Batches that would need segments above kMaxSegment rows take their
+// tasks in turns: in double the shortest segments whose tasks fill the fewest
+// turns, in float kMaxSegment.  us per step with kMaxSegment everywhere -> now
+// (double / float): 8 tiles of 48^2 .. 200^2 61.5 -> 9.9 / 44.3 -> 9.7, 32 of 300^2
+// 61.3 -> 31.3 / 45.6 -> 23.5, 4 of 256^2 .. 1024^2 61.0 -> 20.6 / 44.8 -> 16.4, 32 of
+// 152^2 .. 952^2 98 -> 92 / 67.0 -> 61.7, 20 of 1000^2 194 -> 180 (imaginary time
+// 171 -> 144) / 100 -> 97.
+constexpr int kMaxSegment = 128, kMinSegment = 8;
+
+int auto_segment(const ts_b200_batch *b) {
+    static const double cost[4] = {1.0, 1.32, 1.70, 2.13};
+    const long per = 4L * b->num_sms;  // warps at 4 per SM
+    auto tasks = [&](int rows) {
+        long n = 0;
+        for (const ts_b200_kernel *t : b->k)
+            n += (long)div_up(t->W, kWO) * div_up(t->H, tile_seg_rows(t, rows));
+        return n;
+    };
+    // the fewest rows with at most `most` tasks, 0 above kMaxSegment
+    auto fewest = [&](long most) {
+        for (int rows = kMinSegment; rows <= kMaxSegment; rows += 2)
+            if (tasks(rows) <= most) return rows;
+        return 0;
+    };
+    int best = 0;
+    double least = 0.0;
+    for (int q = 4; q >= 1; --q) {
+        const int rows = fewest(q * per);
+        if (!rows) break;
+        const size_t smem = batch_smem(b, 4, b->walk ? tsb::w2_vlen(rows, false) : 0);
+        if (q * (smem + tsbh::kSmemReservedPerBlock) > tsbh::kSmemPerSm) continue;
+        const double c = (rows + 2 * kHY) * cost[q - 1];
+        if (best == 0 || c < least) {
+            best = rows;
+            least = c;
+        }
+    }
+    if (best) return best;
+    if (!b->fp32)
+        for (long turns = 1; turns <= 8; ++turns)
+            if (const int rows = fewest(turns * 4 * per)) return rows;
+    return kMaxSegment;
 }
 
 void drop_batch_graph(ts_b200_batch *b) {
@@ -210,6 +261,7 @@ cudaError_t launch_batch_kernel<float>(ts_b200_batch *b, const BatchArgs<float> 
 template <typename T>
 int build_layout(ts_b200_batch *b) {
     const int n = (int)b->k.size();
+    if (b->auto_seg) b->shape.seg_rows = auto_segment(b);
     std::vector<int2> tasks;
     std::vector<TileNorm> norms(n);
     std::vector<TileHalo> halos;
@@ -459,6 +511,7 @@ int autotune_t(ts_b200_batch *b, int trial_steps, int use_cache) {
                 b->resident_blocks = 0;
                 b->layout_valid = false;
             }
+            b->auto_seg = false;
             return TS_B200_OK;
         }
     }
@@ -467,6 +520,7 @@ int autotune_t(ts_b200_batch *b, int trial_steps, int use_cache) {
     static const int kSegRows[] = {16, 32, 64, 96, 128, 192, 256};
     static const int kWarps[] = {4, 2};
     constexpr int kShapes = 14;
+    b->auto_seg = false;
     // two passes over the candidates, each keeping its faster time: a clock
     // that moves during the search (power capping) then favours no shape
     float shape_ms[kShapes];
@@ -607,7 +661,10 @@ int ts_b200_batch_set_launch(ts_b200_batch *b, int segment_rows, int warps_per_b
     if (!b || segment_rows < 0) return TS_B200_INVALID_ARGUMENT;
     if (warps_per_block != 0 && warps_per_block != 1 && warps_per_block != 2 && warps_per_block != 4)
         return TS_B200_INVALID_ARGUMENT;
-    if (segment_rows) b->shape.seg_rows = even_up(std::max(2, segment_rows));
+    if (segment_rows) {
+        b->shape.seg_rows = even_up(std::max(2, segment_rows));
+        b->auto_seg = false;
+    }
     if (warps_per_block) b->shape.warps = warps_per_block;
     b->resident_blocks = 0;
     b->layout_valid = false;

@@ -78,6 +78,10 @@ extern std::atomic<uint64_t> g_launches;
 
 inline int div_up(long a, long b) { return (int)((a + b - 1) / b); }
 
+// Shared memory of an SM, and what every block takes of it beyond its own need.
+constexpr int kSmemPerSm = 228 * 1024;
+constexpr int kSmemReservedPerBlock = 1024;
+
 // Entries of the FP32 real-time kinetic coefficient schedule (repeats after).
 constexpr int kSchedLen = 4096;
 

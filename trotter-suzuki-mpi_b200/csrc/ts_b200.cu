@@ -552,9 +552,8 @@ cudaError_t dispatch_step<float>(int C, bool imag, bool rot, int phase, int w2,
 
 using tsbh::div_up;
 
-// Shared memory of an SM and the part the runtime reserves per block (sm_100).
-constexpr int kSmemPerSm = 228 * 1024;
-constexpr int kSmemReservedPerBlock = 1024;
+using tsbh::kSmemPerSm;
+using tsbh::kSmemReservedPerBlock;
 using tsbh::slot_bytes;
 using tsbh::kSchedLen;
 
