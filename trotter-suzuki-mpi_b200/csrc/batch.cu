@@ -8,11 +8,13 @@
 // imaginary time) one reduction block per tile that turns the task partials
 // into the tile's squared norm and renormalisation factor, then (for tiles
 // with periodic boundaries, except on the last step of an evolve) one
-// batched halo refresh.  Runs of 32 steps are replayed from a CUDA graph.
+// batched halo refresh.  Runs of 32 steps are replayed from a CUDA graph.  On the
+// look-ahead walk all of them are programmatic dependent launches.
 //
-// The tile shape (rows per segment task, warps per block) is chosen by a
-// timing autotuner over a small candidate set; the choice is cached per batch
-// signature (precision, time mode, tile sizes) for the process.
+// The rows per segment task are chosen by the tiles' sizes (auto_segment) or, on
+// request, with the warps per block by a timing autotuner over a small candidate
+// set; its choice is cached per batch signature (precision, time mode, tile
+// sizes) for the process.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,8 +57,10 @@ constexpr int kGraphSteps = 32;
 constexpr int kNormThreads = 256;
 
 __global__ void batch_norm_kernel(const TileNorm *tn, const double *task_norm) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const TileNorm n = tn[blockIdx.x];
     __shared__ double red[kNormThreads];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     double s = 0.0;
     for (int i = threadIdx.x; i < n.count; i += blockDim.x) s += task_norm[n.first + i];
     red[threadIdx.x] = s;
@@ -72,17 +76,12 @@ __global__ void batch_norm_kernel(const TileNorm *tn, const double *task_norm) {
     }
 }
 
-// FP32 real time: every tile's coefficient schedule advances by one step
-// (the single-tile kernel's last block does this for its own tile).
-__global__ void batch_step_count_kernel(const TileNorm *tn, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) tn[i].scal->step += 1u;
-}
-
 // blockIdx.y: periodic tile; the x blocks stride over its destination cells.
 template <typename T>
 __global__ void batch_halo_kernel(const StepArgs<T> *inst, const TileHalo *th) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const TileHalo h = th[blockIdx.y];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     Cx<T> *psi = reinterpret_cast<Cx<T> *>(const_cast<void *>(inst[h.tile].psi_out));
     tsb::halo_cells(psi, h.W, h.H, h.P, h.hx, h.hy, h.px, h.py, h.iy0, h.iy0 + h.H - 2 * h.hy,
                     blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
@@ -120,7 +119,7 @@ struct ts_b200_batch {
     TileNorm *d_norm = nullptr;
     TileHalo *d_halo = nullptr;
     int n_halo = 0, halo_cells_max = 0;
-    int *d_error = nullptr;
+    int *d_error = nullptr;       // and the launches' block count
     std::vector<int> args_cur;    // cur of each tile the argument tables were built for
     bool layout_valid = false;
     cudaStream_t own_stream = nullptr, stream = nullptr;
@@ -231,29 +230,39 @@ void drop_batch_graph(ts_b200_batch *b) {
     }
 }
 
+// Shared memory of a launch whose next one's blocks are placed early: enough
+// that no SM holds more blocks of both than this grid's share (as geometry in
+// ts_b200.cu).
+size_t launch_smem(const ts_b200_batch *b, int blocks) {
+    const size_t smem = batch_smem(b, b->shape.warps);
+    if (!b->walk || blocks == 0) return smem;
+    const int per_sm = div_up(blocks, b->num_sms);
+    return std::max(smem, (size_t)tsbh::kSmemPerSm / (per_sm + 1) - tsbh::kSmemReservedPerBlock + 128);
+}
+
 template <typename T>
 cudaError_t launch_batch_kernel(ts_b200_batch *b, const BatchArgs<T> &a, int blocks, int *bps);
 
 template <>
 cudaError_t launch_batch_kernel<double>(ts_b200_batch *b, const BatchArgs<double> &a, int blocks,
                                         int *bps) {
-    const size_t smem = batch_smem(b, b->shape.warps);
+    const size_t smem = launch_smem(b, blocks);
     if (b->walk)
         return b->imag ? tsb::launch_batch2_f64_imag(b->phase, a, b->shape.warps, smem, blocks,
-                                                     b->stream, bps)
+                                                     b->stream, bps, true)
                        : tsb::launch_batch2_f64_real(b->phase, a, b->shape.warps, smem, blocks,
-                                                     b->stream, bps);
+                                                     b->stream, bps, true);
     return tsb::launch_batch_f64(b->imag, b->phase, a, b->shape.warps, smem, blocks, b->stream, bps);
 }
 template <>
 cudaError_t launch_batch_kernel<float>(ts_b200_batch *b, const BatchArgs<float> &a, int blocks,
                                        int *bps) {
-    const size_t smem = batch_smem(b, b->shape.warps);
+    const size_t smem = launch_smem(b, blocks);
     if (b->walk)
         return b->imag ? tsb::launch_batch2_f32_imag(b->phase, a, b->shape.warps, smem, blocks,
-                                                     b->stream, bps)
+                                                     b->stream, bps, true)
                        : tsb::launch_batch2_f32_real(b->phase, a, b->shape.warps, smem, blocks,
-                                                     b->stream, bps);
+                                                     b->stream, bps, true);
     return tsb::launch_batch_f32(b->imag, b->phase, a, b->shape.warps, smem, blocks, b->stream, bps);
 }
 
@@ -352,6 +361,21 @@ int build_args(ts_b200_batch *b) {
     return TS_B200_OK;
 }
 
+// A launch on the batch's stream with programmatic dependent launch.
+template <typename... A>
+cudaError_t launch_dependent(ts_b200_batch *b, void (*fn)(A...), dim3 grid, int threads, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = b->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = b->walk ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 // One step of every tile: parity p selects the argument table.
 template <typename T>
 int launch_batch_step(ts_b200_batch *b, int p, bool exchange, bool renorm_pass = true) {
@@ -360,6 +384,8 @@ int launch_batch_step(ts_b200_batch *b, int p, bool exchange, bool renorm_pass =
     a.tasks = b->d_tasks;
     a.task_norm = b->d_task_norm;
     a.error = b->d_error;
+    a.ticket = reinterpret_cast<unsigned int *>(b->d_error + 1);
+    a.n_tiles = b->fp32 && !b->imag && renorm_pass ? (int)b->k.size() : 0;
     a.n_tasks = b->n_tasks;
     a.ring = b->ring;
     a.vlen = b->walk ? batch_vlen(b) : 0;
@@ -367,25 +393,18 @@ int launch_batch_step(ts_b200_batch *b, int p, bool exchange, bool renorm_pass =
     cudaError_t e = launch_batch_kernel<T>(b, a, blocks, nullptr);
     if (e != cudaSuccess) return bcuda(b, e, "batch step launch");
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    if (b->fp32 && !b->imag && renorm_pass) {
-        const int n = (int)b->k.size();
-        batch_step_count_kernel<<<div_up(n, 256), 256, 0, b->stream>>>(b->d_norm, n);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return bcuda(b, e, "batch step count launch");
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-    }
     if (b->imag && renorm_pass) {
-        batch_norm_kernel<<<(unsigned)b->k.size(), kNormThreads, 0, b->stream>>>(b->d_norm,
-                                                                               b->d_task_norm);
-        e = cudaGetLastError();
+        e = launch_dependent(b, batch_norm_kernel, dim3((unsigned)b->k.size()), kNormThreads,
+                             static_cast<const TileNorm *>(b->d_norm),
+                             static_cast<const double *>(b->d_task_norm));
         if (e != cudaSuccess) return bcuda(b, e, "batch norm launch");
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
     if (exchange && b->n_halo > 0) {
         const unsigned gx = (unsigned)std::max(1, std::min(div_up(b->halo_cells_max, 256), 1024));
-        batch_halo_kernel<T><<<dim3(gx, (unsigned)b->n_halo), 256, 0, b->stream>>>(
-            static_cast<const StepArgs<T> *>(b->d_args[p]), b->d_halo);
-        e = cudaGetLastError();
+        e = launch_dependent(b, batch_halo_kernel<T>, dim3(gx, (unsigned)b->n_halo), 256,
+                             static_cast<const StepArgs<T> *>(b->d_args[p]),
+                             static_cast<const TileHalo *>(b->d_halo));
         if (e != cudaSuccess) return bcuda(b, e, "batch halo launch");
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
@@ -393,7 +412,7 @@ int launch_batch_step(ts_b200_batch *b, int p, bool exchange, bool renorm_pass =
 }
 
 int kernels_per_batch_step(const ts_b200_batch *b, bool exchange) {
-    return 1 + ((b->imag || b->fp32) ? 1 : 0) + ((exchange && b->n_halo > 0) ? 1 : 0);
+    return 1 + (b->imag ? 1 : 0) + ((exchange && b->n_halo > 0) ? 1 : 0);
 }
 
 // The batch stream waits for every tile's queued work, or the tiles' streams
@@ -608,8 +627,8 @@ int ts_b200_batch_create(ts_b200_kernel *const *kernels, int n, ts_b200_batch **
     for (int p = 0; p < 2 && e == cudaSuccess; ++p) e = cudaMalloc(&b->d_args[p], n * b->args_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_norm, n * sizeof(TileNorm));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_halo, n * sizeof(TileHalo));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_error, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(b->d_error, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_error, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(b->d_error, 0, 2 * sizeof(int));
     if (e != cudaSuccess) {
         const int st = e == cudaErrorMemoryAllocation ? TS_B200_OUT_OF_MEMORY : TS_B200_CUDA_ERROR;
         ts_b200_batch_destroy(b);

@@ -4,8 +4,8 @@
 namespace tsb {
 
 cudaError_t launch_batch2_f64_real(int phase, const BatchArgs<double> &b, int warps, size_t smem,
-                                   int blocks, cudaStream_t st, int *bps) {
-    return launch_batch2_t<double, false>(phase, b, warps, smem, blocks, st, bps);
+                                   int blocks, cudaStream_t st, int *bps, bool pdl) {
+    return launch_batch2_t<double, false>(phase, b, warps, smem, blocks, st, bps, pdl);
 }
 
 }  // namespace tsb

@@ -8,7 +8,7 @@ namespace tsb {
 
 template <class V>
 cudaError_t launch_batch2_variant(const BatchArgs<typename V::T> &b, int warps, size_t smem,
-                                  int blocks, cudaStream_t st, int *blocks_per_sm) {
+                                  int blocks, cudaStream_t st, int *blocks_per_sm, bool pdl) {
     auto fn = batch2_kernel<V, 2>;
     static int configured_smem = -1;
     if ((int)smem > configured_smem) {
@@ -23,16 +23,25 @@ cudaError_t launch_batch2_variant(const BatchArgs<typename V::T> &b, int warps, 
         if (e != cudaSuccess) return e;
     }
     if (blocks == 0) return cudaSuccess;
-    fn<<<blocks, warps * 32, smem, st>>>(b);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, b);
 }
 
 template <typename T, bool IMAG>
 cudaError_t launch_batch2_t(int phase, const BatchArgs<T> &b, int warps, size_t smem, int blocks,
-                            cudaStream_t st, int *bps) {
-    if (phase == 2) return launch_batch2_variant<Variant<T, 2, IMAG, false, 2>>(b, warps, smem, blocks, st, bps);
-    if (phase == 1) return launch_batch2_variant<Variant<T, 2, IMAG, false, 1>>(b, warps, smem, blocks, st, bps);
-    return launch_batch2_variant<Variant<T, 2, IMAG, false, 0>>(b, warps, smem, blocks, st, bps);
+                            cudaStream_t st, int *bps, bool pdl) {
+    if (phase == 2) return launch_batch2_variant<Variant<T, 2, IMAG, false, 2>>(b, warps, smem, blocks, st, bps, pdl);
+    if (phase == 1) return launch_batch2_variant<Variant<T, 2, IMAG, false, 1>>(b, warps, smem, blocks, st, bps, pdl);
+    return launch_batch2_variant<Variant<T, 2, IMAG, false, 0>>(b, warps, smem, blocks, st, bps, pdl);
 }
 
 }  // namespace tsb

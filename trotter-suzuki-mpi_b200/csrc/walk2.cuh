@@ -974,12 +974,15 @@ template <class V, int R>
 __global__ void __launch_bounds__(128, 4) batch2_kernel(BatchArgs<typename V::T> b) {
     using T = typename V::T;
     extern __shared__ __align__(128) unsigned char smem[];
+    // as step2_kernel: the next launch's set-up overlaps this one's tail
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warps = blockDim.x >> 5;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
     Walk2<V, R> w;
     w2_warp_setup(w, smem, warps, warp, lane, b.vlen);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int t = blockIdx.x * warps + warp; t < b.n_tasks && !w.failed; t += gridDim.x * warps) {
         const int2 it = __ldg(&b.tasks[t]);
         const int tile = bcast0(it.x), task = bcast0(it.y);
@@ -995,6 +998,7 @@ __global__ void __launch_bounds__(128, 4) batch2_kernel(BatchArgs<typename V::T>
         }
     }
     if (w.failed && lane == 0) atomicExch(b.error, 1);
+    batch_count_steps<V>(b);
 }
 
 }  // namespace tsb
