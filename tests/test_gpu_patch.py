@@ -235,6 +235,48 @@ def test_adjoint_patches_match_the_row_walk(N, Ny, g, lhy, every, imag):
         _close(got, old, imag)
 
 
+@pytest.mark.parametrize("W,H,pad,shift", [(1, 1, 0, 0), (5, 3, 2, 0), (1023, 2, 1, 1),
+                                           (1025, 7, 0, 0), (2050, 3, 3, 1), (31, 300, 0, 1)])
+@pytest.mark.parametrize("precision,imag", [(0, False), (0, True), (1, False), (1, True)])
+def test_device_state_and_table_copies(W, H, pad, shift, precision, imag):
+    """States and tables from and to device rows of any pitch; shift: rows that
+    start half an element off its alignment (states in real time only go in)."""
+    import torch
+    from trottersuzuki_b200 import Kernel
+    lat, psi0, V = seeded_case(W, 0.2 * W, H)
+    p = lat.params(1e-3, imag, 1.0, 1.0, 0.0, norm0=1.0 if imag else 0.0)
+    real = torch.float32 if precision else torch.float64
+    ctype = torch.complex64 if precision else torch.complex128
+    k = Kernel(desc_from_params(p, precision=precision))
+
+    def rows(a, n):  # n reals per element, `shift` reals into an allocation
+        flat = torch.zeros(H * (W + pad) * n + shift, dtype=real, device="cuda")
+        r = flat[shift:].view(H, W + pad, n)
+        r[:, :W] = a
+        return r
+
+    src = torch.tensor(psi0, device="cuda").to(ctype)
+    r = rows(torch.view_as_real(src), 2)
+    k.set_state_device(r.data_ptr(), W + pad)
+    out = torch.full((H, W + pad), 7.0, dtype=ctype, device="cuda")
+    k.get_state_device(out.data_ptr(), W + pad)
+    assert torch.equal(out[:, :W], src)
+    assert bool((out[:, W:] == 7).all())
+    k.close()
+    # the table: the same step as with whole rows side by side
+    tab = torch.tensor(np.exp((-1e-3 if imag else -1e-3j) * V), device="cuda")
+    tab = tab.to(real)[..., None] if imag else torch.view_as_real(tab.to(ctype))
+    n = tab.shape[-1]
+    steps = []
+    for r, pitch in ((rows(tab, n), W + pad), (tab.contiguous(), W)):
+        with Kernel(desc_from_params(p, precision=precision)) as k:
+            k.set_state_device(src.data_ptr(), W)
+            k.set_exp_potential_device(r.data_ptr(), pitch)
+            k.step(exchange=False)
+            steps.append(k.get_state())
+    assert np.array_equal(*steps, equal_nan=True)
+
+
 def test_asking_for_a_walk_or_overlap_after_steps_keeps_the_evolution():
     """Switches of walk and launch mode between evolve calls that replay graphs."""
     from trottersuzuki_b200 import Kernel

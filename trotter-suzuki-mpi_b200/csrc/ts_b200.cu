@@ -247,22 +247,57 @@ __global__ void unpack_state_kernel(const Cx<T> *src, int P, int x0, int y0, int
     }
 }
 
-// Copy the tile with a pitch change, optionally folding in the pending scale.
-template <typename T>
-__global__ void copy_tile_kernel(Cx<T> *dst, size_t dpitch, const Cx<T> *src, size_t spitch,
-                                 int W, int H, const Scalars *scal, int use_scale) {
-    const T s = use_scale ? (T)scal->pending_inv : T(1);
-    const size_t n = (size_t)W * H;
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
-         k += (size_t)gridDim.x * blockDim.x) {
-        const int y = (int)(k / W), x = (int)(k % W);
-        Cx<T> v = src[(size_t)y * spitch + x];
-        if (use_scale) {
-            v.re *= s;
-            v.im *= s;
-        }
-        dst[(size_t)y * dpitch + x] = v;
+// Copies of a tile with a pitch change, bound by memory: 4 cells in flight per
+// thread, no division per cell (2048^2 double 20.9 us, 8192^2 float 158: 6.4 and
+// 6.8 TB/s; cudaMemcpy2DAsync 72 and 545, a cell per thread and turn 24.9 and
+// 209).
+constexpr int kCopyThreads = 256, kCopyCells = 4;
+
+// H rows of W units; reset: the pending renormalisation becomes 1 (a state from
+// outside carries none).
+template <typename U>
+__global__ void __launch_bounds__(kCopyThreads)
+    copy_rows_kernel(U *dst, size_t dpitch, const U *src, size_t spitch, int W, int H,
+                     Scalars *reset) {
+    const int x = blockIdx.x * kCopyThreads * kCopyCells + threadIdx.x;
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const U *s = src + (size_t)y * spitch + x;
+        U *d = dst + (size_t)y * dpitch + x;
+        U v[kCopyCells];
+#pragma unroll
+        for (int i = 0; i < kCopyCells; ++i)
+            if (x + i * kCopyThreads < W) v[i] = s[i * kCopyThreads];
+#pragma unroll
+        for (int i = 0; i < kCopyCells; ++i)
+            if (x + i * kCopyThreads < W) d[i * kCopyThreads] = v[i];
     }
+    if (reset && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) reset->pending_inv = 1.0;
+}
+
+// The same with the pending renormalisation multiplied in.
+template <typename T>
+__global__ void __launch_bounds__(kCopyThreads)
+    scale_rows_kernel(Cx<T> *dst, size_t dpitch, const Cx<T> *src, size_t spitch, int W, int H,
+                      const Scalars *scal) {
+    const T f = (T)scal->pending_inv;
+    const int x = blockIdx.x * kCopyThreads * kCopyCells + threadIdx.x;
+    for (int y = blockIdx.y; y < H; y += gridDim.y) {
+        const Cx<T> *s = src + (size_t)y * spitch + x;
+        Cx<T> *d = dst + (size_t)y * dpitch + x;
+        Cx<T> v[kCopyCells];
+#pragma unroll
+        for (int i = 0; i < kCopyCells; ++i)
+            if (x + i * kCopyThreads < W) v[i] = s[i * kCopyThreads];
+#pragma unroll
+        for (int i = 0; i < kCopyCells; ++i)
+            if (x + i * kCopyThreads < W)
+                d[i * kCopyThreads] = Cx<T>{v[i].re * f, v[i].im * f};
+    }
+}
+
+dim3 copy_grid(int W, int H) {
+    return dim3((unsigned)((W + kCopyThreads * kCopyCells - 1) / (kCopyThreads * kCopyCells)),
+                (unsigned)std::min(H, 65535));
 }
 
 // Periodic halo refresh (src/cpukernel.cpp:706-716,738-746, one process):
@@ -1341,6 +1376,33 @@ int upload_kinetic_schedule(ts_b200_kernel *k) {
 
 int grid_for(size_t n) { return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 8192)); }
 
+// Rows of W elements of `cell` bytes (4, 8 or 16), pitches in elements, on the
+// handle's stream; what is not aligned to an element goes through the runtime.
+int copy_rows(ts_b200_kernel *k, void *dst, size_t dpitch, const void *src, size_t spitch,
+              size_t cell, Scalars *reset) {
+    const dim3 grid = copy_grid(k->W, k->H);
+    if (((uintptr_t)dst | (uintptr_t)src) % cell != 0) {
+        TSB_CHECK(k, cudaMemcpy2DAsync(dst, dpitch * cell, src, spitch * cell, k->W * cell, k->H,
+                                       cudaMemcpyDeviceToDevice, k->stream));
+        const double one = 1.0;
+        if (reset)
+            TSB_CHECK(k, cudaMemcpyAsync(&reset->pending_inv, &one, sizeof(double),
+                                         cudaMemcpyHostToDevice, k->stream));
+        return TS_B200_OK;
+    }
+    auto run = [&](auto unit) {
+        using U = decltype(unit);
+        copy_rows_kernel<U><<<grid, kCopyThreads, 0, k->stream>>>(
+            static_cast<U *>(dst), dpitch, static_cast<const U *>(src), spitch, k->W, k->H, reset);
+    };
+    if (cell == 16) run(uint4{});
+    else if (cell == 8) run(uint2{});
+    else run(0u);
+    TSB_CHECK(k, cudaGetLastError());
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return TS_B200_OK;
+}
+
 // The pending factor from a norm summed over several tiles (one lattice
 // split across ranks): src/cpukernel.cpp:537-562 with the MPI_Allgather sum.
 __global__ void renorm_from_kernel(Scalars *scal, const double *total, double norm0) {
@@ -1600,27 +1662,21 @@ int ts_b200_set_exp_potential(ts_b200_kernel *k, const double *re, const double 
 
 int ts_b200_set_state_device(ts_b200_kernel *k, const void *aos, size_t pitch) {
     if (!k || !aos || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    TSB_CHECK(k, cudaMemcpy2DAsync(k->psi[k->cur], k->P * k->cell, aos, pitch * k->cell,
-                                   k->W * k->cell, k->H, cudaMemcpyDeviceToDevice, k->stream));
-    const double one = 1.0;
-    TSB_CHECK(k, cudaMemcpyAsync(&k->scal->pending_inv, &one, sizeof(double), cudaMemcpyHostToDevice,
-                                 k->stream));
-    return TS_B200_OK;
+    return copy_rows(k, k->psi[k->cur], k->P, aos, pitch, k->cell, k->scal);
 }
 
 int ts_b200_get_state_device(ts_b200_kernel *k, void *aos, size_t pitch) {
     if (!k || !aos || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    const size_t n = (size_t)k->W * k->H;
+    if (!k->imag) return copy_rows(k, aos, pitch, k->psi[k->cur], k->P, k->cell, nullptr);
+    const dim3 grid = copy_grid(k->W, k->H);
     if (k->fp32)
-        copy_tile_kernel<float><<<grid_for(n), 256, 0, k->stream>>>(
-            reinterpret_cast<Cx<float> *>(aos), pitch,
-            reinterpret_cast<const Cx<float> *>(k->psi[k->cur]), k->P, k->W, k->H, k->scal,
-            k->imag ? 1 : 0);
+        scale_rows_kernel<float><<<grid, kCopyThreads, 0, k->stream>>>(
+            static_cast<Cx<float> *>(aos), pitch, static_cast<const Cx<float> *>(k->psi[k->cur]),
+            k->P, k->W, k->H, k->scal);
     else
-        copy_tile_kernel<double><<<grid_for(n), 256, 0, k->stream>>>(
-            reinterpret_cast<Cx<double> *>(aos), pitch,
-            reinterpret_cast<const Cx<double> *>(k->psi[k->cur]), k->P, k->W, k->H, k->scal,
-            k->imag ? 1 : 0);
+        scale_rows_kernel<double><<<grid, kCopyThreads, 0, k->stream>>>(
+            static_cast<Cx<double> *>(aos), pitch, static_cast<const Cx<double> *>(k->psi[k->cur]),
+            k->P, k->W, k->H, k->scal);
     TSB_CHECK(k, cudaGetLastError());
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return TS_B200_OK;
@@ -1628,9 +1684,7 @@ int ts_b200_get_state_device(ts_b200_kernel *k, void *aos, size_t pitch) {
 
 int ts_b200_set_exp_potential_device(ts_b200_kernel *k, const void *table, size_t pitch) {
     if (!k || !table || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    TSB_CHECK(k, cudaMemcpy2DAsync(k->tab, k->P * k->tab_cell, table, pitch * k->tab_cell,
-                                   k->W * k->tab_cell, k->H, cudaMemcpyDeviceToDevice, k->stream));
-    return TS_B200_OK;
+    return copy_rows(k, k->tab, k->P, table, pitch, k->tab_cell, nullptr);
 }
 
 int ts_b200_set_potential_device(ts_b200_kernel *k, const double *potential, size_t pitch,
