@@ -10,7 +10,10 @@
 // horizontal ones shuffles between the warp's two columns and an exchange
 // through shared memory between warps (two buffers in turn, one block barrier
 // per horizontal sweep).  The arithmetic of a cell is that of the row walks
-// (the same pair forms and potential row), so all give the same bits.
+// (the same pair forms and potential row): in real time the bits are theirs.  Two
+// things depend on how a tile is cut: the order of the norm's sum in imaginary
+// time, and the warp's choice of a nonlinear phase's evaluation in imaginary time
+// and in a double rotating frame, once phases pass 2^-8 (step_kernel.cuh).
 //
 // Against the look-ahead walk (walk2.cuh) a step is one load, nine stages of
 // a region and one store instead of a chain of nine stages per row: what a

@@ -504,68 +504,81 @@ __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 // Phase factors of the GPE / LHY term for small arguments.  The nonlinear
 // phase g*dt*|psi|^2 is far below 1/32 in practice, where truncated Maclaurin
 // series of cos, sin and exp (Horner's rule) leave a remainder well under half
-// an ulp; larger arguments take the CUDA math library.  Two tiers:
-//   |th| < 2^-8: double cos / sin to the t^3 terms (t = th^2), exp to x^6
+// an ulp; larger arguments take the CUDA math library.  Tiers:
+//   double, |th| < 2^-8: cos / sin to the t^3 terms (t = th^2), exp to x^6
 //                (remainders below 3e-21; Estrin's scheme, a shorter
-//                dependency chain than Horner's); float cos / sin to t^2,
-//                exp to x^4 (below 1e-14);
-//   |th| < 1/32: cos / sin to t^5, exp to x^8 (remainders below 1e-19).
-// The warp takes the shortest that serves all its cells, or (CELL, sin and
-// cos) each cell its own: a warp whose cells are all in the first tier, the
-// usual case, evaluates that one only, another the second, and the cells in
-// the first tier or past the second replace its result.  With two branches
-// instead of three for the whole warp more of the row body is scheduled
-// across them: the 2048^2 double real-time step took 38.7 us against
-// 43.9-48.0 (phases of the second tier 46.6 / 49.7, of the library 65.2 /
-// 63.6).  Float gains nothing by it (25.5 / 25.9; library 47.7 / 43.7) and
-// keeps the warp's choice.  REST: that choice with all but the first tier in
-// a function of its own, for the rotating frame, whose row body is bound by
-// instruction fetch (float 4096^2 151.3 -> 143.2 us, 2300^2 67.6 -> 62.9,
-// double 1400^2 46.1 -> 44.0, 2048^2 76.6 -> 75.5, 4096^2 291.8 -> 288.5, 3000^2
-// 140.2 -> 142; float with phases of the second tier 154.1 -> 164.4, of the
-// library 225 -> 234).  Returns sin(th) and cos(th) (cos(th) - 1 in delta form).
-// The comparisons are exact in either precision.
+//                dependency chain than Horner's);
+//   double, |th| < 1/32: cos / sin to t^5, exp to x^8 (remainders below 1e-19);
+//   float, |th| < 1/32: cos - 1 and sin to t^2 (sincos_series);
+//   float exp: to x^4 below 2^-8 (1e-14), to x^8 below 1/32.
+// sin and cos of a cell follow from its own argument alone in float and, outside
+// the rotating frame, in double: however a tile is cut into warps, regions and
+// launches, its cells keep their bits.  In a double rotating frame the warp takes
+// the tier that serves all its cells.
+// Double: a warp whose cells are all in the first tier, the usual case,
+// evaluates that one only, another the second, and the cells in the first tier
+// or past the second replace its result.  With two branches instead of three
+// for the whole warp more of the row body is scheduled across them: the 2048^2
+// double real-time step took 38.7 us against 43.9-48.0 (phases of the second
+// tier 46.6 / 49.7, of the library 65.2 / 63.6).
+// ROT: all but the first path in a function of its own, for the rotating frame,
+// whose row body is bound by instruction fetch.  Double, against the same tiers
+// in line: 1500^2 50.3 -> 47.8 us, 2048^2 76.6 -> 75.6, 3000^2 139.0 -> 138.8, 4096^2
+// 296.8 -> 293.4; 4096^2 with phases of the second tier 361 -> 375, of the library
+// 398 -> 409.
+// Float, against two series and the library by the warp's choice (first tier /
+// second / library): 1200^2 12.8 / 13.6 / 22.9 -> 11.6 / 11.8 / 21.8, 2048^2 26.1
+// / 28.0 / 44.2 -> 24.9 / 25.1 / 41.8; rotating frame 4096^2 142.5 / 179.8 / 235
+// -> 143.2 / 177.9 / 216, 8192^2 547 / 652 / 979 -> 549 / 552 / 871 (in line, as
+// elsewhere in float, 565 / 557 / 857).
+// Returns sin(th) and cos(th) (cos(th) - 1 in delta form).  The comparisons are
+// exact in either precision.
 __device__ __forceinline__ bool phase_tiny(double th) { return fabs(th) < 0.00390625; }
 __device__ __forceinline__ bool phase_tiny(float th) { return fabsf(th) < 0.00390625f; }
 __device__ __forceinline__ bool phase_small(double th) { return fabs(th) < 0.03125; }
 __device__ __forceinline__ bool phase_small(float th) { return fabsf(th) < 0.03125f; }
 
-template <typename T>
-__device__ __forceinline__ void sincos_tiny(T th, T *s, T *c) {
-    const T t = th * th;
-    if constexpr (std::is_same<T, float>::value) {
-        const T pc = fma_t(T(4.1666666666666664e-02), t, T(-0.5));               // 1/4!, -1/2!
-        const T ps = fma_t(T(8.3333333333333332e-03), t, T(-1.6666666666666666e-01));  // 1/5!, -1/3!
-        *c = DeltaForm<T>::value ? mul_t(pc, t) : fma_t(pc, t, T(1));
-        *s = fma_t(mul_t(ps, t), th, th);
-    } else {
-        // Estrin's scheme (two levels instead of Horner's three):
-        // cos = (1 - t/2!) + t^2 (1/4! - t/6!),
-        // sin = th + (th t) ((-1/3! + t/5!) - t^2/7!)
-        const T t2 = mul_t(t, t);
-        const T c0 = fma_t(t, T(-0.5), T(1));
-        const T c1 = fma_t(t, T(-1.3888888888888889e-03), T(4.1666666666666664e-02));
-        const T s0 = fma_t(t, T(8.3333333333333332e-03), T(-1.6666666666666666e-01));
-        const T ps = fma_t(t2, T(-1.9841269841269841e-04), s0);
-        *c = fma_t(c1, t2, c0);
-        *s = fma_t(mul_t(th, t), ps, th);
-    }
+// |th| < 2^-8, Estrin's scheme (two levels instead of Horner's three):
+// cos = (1 - t/2!) + t^2 (1/4! - t/6!),
+// sin = th + (th t) ((-1/3! + t/5!) - t^2/7!)
+__device__ __forceinline__ void sincos_tiny(double th, double *s, double *c) {
+    const double t = th * th;
+    const double t2 = mul_t(t, t);
+    const double c0 = fma_t(t, -0.5, 1.0);
+    const double c1 = fma_t(t, -1.3888888888888889e-03, 4.1666666666666664e-02);
+    const double s0 = fma_t(t, 8.3333333333333332e-03, -1.6666666666666666e-01);
+    const double ps = fma_t(t2, -1.9841269841269841e-04, s0);
+    *c = fma_t(c1, t2, c0);
+    *s = fma_t(mul_t(th, t), ps, th);
 }
 
-template <typename T>
-__device__ __forceinline__ void sincos_small(T th, T *s, T *c) {
-    const T t = th * th;
-    T pc = T(-2.7557319223985893e-07);            // -1/10!
-    pc = fma_t(pc, t, T(2.4801587301587302e-05));  //  1/8!
-    pc = fma_t(pc, t, T(-1.3888888888888889e-03)); // -1/6!
-    pc = fma_t(pc, t, T(4.1666666666666664e-02));  //  1/4!
-    pc = fma_t(pc, t, T(-0.5));                    // -1/2!
-    T ps = T(-2.5052108385441720e-08);             // -1/11!
-    ps = fma_t(ps, t, T(2.7557319223985888e-06));  //  1/9!
-    ps = fma_t(ps, t, T(-1.9841269841269841e-04)); // -1/7!
-    ps = fma_t(ps, t, T(8.3333333333333332e-03));  //  1/5!
-    ps = fma_t(ps, t, T(-1.6666666666666666e-01)); // -1/3!
-    *c = DeltaForm<T>::value ? mul_t(pc, t) : fma_t(pc, t, T(1));
+// |th| < 1/32
+__device__ __forceinline__ void sincos_small(double th, double *s, double *c) {
+    const double t = th * th;
+    double pc = -2.7557319223985893e-07;             // -1/10!
+    pc = fma_t(pc, t, 2.4801587301587302e-05);       //  1/8!
+    pc = fma_t(pc, t, -1.3888888888888889e-03);      // -1/6!
+    pc = fma_t(pc, t, 4.1666666666666664e-02);       //  1/4!
+    pc = fma_t(pc, t, -0.5);                         // -1/2!
+    double ps = -2.5052108385441720e-08;             // -1/11!
+    ps = fma_t(ps, t, 2.7557319223985888e-06);       //  1/9!
+    ps = fma_t(ps, t, -1.9841269841269841e-04);      // -1/7!
+    ps = fma_t(ps, t, 8.3333333333333332e-03);       //  1/5!
+    ps = fma_t(ps, t, -1.6666666666666666e-01);      // -1/3!
+    *c = fma_t(pc, t, 1.0);
+    *s = fma_t(mul_t(ps, t), th, th);
+}
+
+// Float, |th| < 1/32: sin to t^2, cos - 1 = t (-1/2 + k t).  With k = 1/4! the
+// remainder t^2 / 720 is 2.6e-9 of cos - 1 at 1/32; k = 1/4! - 2 (sqrt(2) - 1) T /
+// 720, T = 2^-10, spreads it evenly over t < T (4.5e-10), so that the errors are
+// those of the longer series (largest 1.43e-7 of cos - 1 with either, mean
+// 3.13e-8).
+__device__ __forceinline__ void sincos_series(float th, float *s, float *c) {
+    const float t = th * th;
+    const float pc = fma_t(4.1665543040466650e-02f, t, -0.5f);
+    const float ps = fma_t(8.3333333333333332e-03f, t, -1.6666666666666666e-01f);  // 1/5!, -1/3!
+    *c = DeltaForm<float>::value ? mul_t(pc, t) : fma_t(pc, t, 1.0f);
     *s = fma_t(mul_t(ps, t), th, th);
 }
 
@@ -579,29 +592,52 @@ __device__ __forceinline__ void sincos_large(T th, T *s, T *c) {
     }
 }
 
-template <typename T>
-static __device__ __noinline__ void sincos_rest(T th, T *s, T *c) {
+// The cells of a warp from 1/32 on take the library, the others keep the series.
+static __device__ __noinline__ void sincos_rest(float th, float *s, float *c) {
+    float s1, c1;
+    sincosf(th, &s1, &c1);
+    if (DeltaForm<float>::value) {
+        const float h = sinf(0.5f * th);
+        c1 = -2.0f * h * h;
+    }
+    sincos_series(th, s, c);
+    const bool small = phase_small(th);
+    *s = small ? *s : s1;
+    *c = small ? *c : c1;
+}
+static __device__ __noinline__ void sincos_rest(double th, double *s, double *c) {
     if (!__any_sync(0xffffffffu, !phase_small(th))) sincos_small(th, s, c);
     else sincos_large(th, s, c);
 }
 
-// TIERS = false: the 1/32 tier and the library only (less code, for the
-// kernels whose row body is long enough for instruction fetch to limit them).
-template <typename T, bool TIERS = true, bool CELL = std::is_same<T, double>::value,
-          bool REST = false>
-__device__ __forceinline__ void phase_sincos(T th, T *s, T *c) {
+// TIERS = false: double without the first tier (less code, for the kernels
+// whose row body is long enough for instruction fetch to limit them).
+template <bool TIERS = true, bool ROT = false>
+__device__ __forceinline__ void phase_sincos(float th, float *s, float *c) {
+    if constexpr (ROT) {
+        if (!__any_sync(0xffffffffu, !phase_small(th))) sincos_series(th, s, c);
+        else sincos_rest(th, s, c);
+    } else {
+        sincos_series(th, s, c);
+        if (__any_sync(0xffffffffu, !phase_small(th))) {
+            float s1, c1;
+            sincos_large(th, &s1, &c1);
+            const bool small = phase_small(th);
+            *s = small ? *s : s1;
+            *c = small ? *c : c1;
+        }
+    }
+}
+template <bool TIERS = true, bool ROT = false>
+__device__ __forceinline__ void phase_sincos(double th, double *s, double *c) {
     if (TIERS && !__any_sync(0xffffffffu, !phase_tiny(th))) {
         sincos_tiny(th, s, c);
-    } else if (REST) {
+    } else if (ROT) {
         sincos_rest(th, s, c);
-    } else if (CELL) {
+    } else {
         sincos_small(th, s, c);
         if (TIERS && phase_tiny(th)) sincos_tiny(th, s, c);
         else if (!phase_small(th)) sincos_large(th, s, c);
-    } else if (!__any_sync(0xffffffffu, !phase_small(th))) {
-        sincos_small(th, s, c);
-    } else {
-        sincos_large(th, s, c);
     }
 }
 
@@ -804,8 +840,7 @@ __device__ __forceinline__ void potential_row(Cx<T> (&w)[C], const TabT *tab, T 
                 T th = mul_t(ca, n2);
                 if (LHY) th = fma_t(caa, mul_t(n2, sqrt_t(n2)), th);
                 if (PB) th = th + thb;
-                constexpr bool F32 = std::is_same<T, float>::value;
-                phase_sincos<T, TIERS, !F32 && !ROT, ROT>(th, &s, &c);
+                phase_sincos<TIERS, ROT>(th, &s, &c);
             }
             // the table holds (cos, sin) of -dt V; in delta form (cos - 1, sin):
             // v (cos + i sin), the kinetic pair's form with the cell as its own
