@@ -206,3 +206,19 @@ def test_rotating_frame_segments_and_fp32(imag, seg):
             assert np.abs(got - old).max() <= (1e-13 if prec == _capi.FP64 else 1e-6) * np.abs(old).max()
         else:
             assert np.array_equal(got, old)
+
+
+@pytest.mark.parametrize("imag,precision", [(False, 0), (True, 0), (True, 1)])
+def test_wide_tiles_take_segments_for_the_blocks_they_fill(imag, precision):
+    """50000 columns are 893 strips: as whole strips 224 blocks of 4 warps, 2 on the
+    fullest of 148 SMs, where 118 rows cost 1.32 each; in two segments 447 blocks, 4
+    on the fullest, and 64 rows at 2.13."""
+    from trottersuzuki_b200 import Kernel
+    lat, psi0, V = seeded_case(50000, 50.0, 110)
+    p = lat.params(1e-9, imag, 1.0, 0.0, 0.0, norm0=1.0 if imag else 0.0)
+    with Kernel(desc_from_params(p, precision)) as k:
+        k.set_state(psi0)
+        k.set_exp_potential(*O.exp_table(V, 1e-9, imag))
+        k.evolve(1)
+        shape = k.launch_shape()
+        assert (shape["walk"], shape["strips"], shape["segments"]) == (2, 893, 2)

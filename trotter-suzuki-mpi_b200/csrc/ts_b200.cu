@@ -676,13 +676,14 @@ int eff_seg(const ts_b200_kernel *k) { return use_walk2(k) ? (k->seg_h + 1) & ~1
 // Rows per segment for a grid of `blocks_per_sm` blocks on every SM, one
 // task per warp: every SM then holds the same number of tasks (the launch
 // time is that of the most loaded SM).
-int balanced_segments(const ts_b200_kernel *k, int blocks_per_sm, int warps) {
+int walk_strips(const ts_b200_kernel *k, int W) {
     const int hx = (k->rot || k->cyl) ? 8 : 4;  // Variant::HX
-    const int wo = 32 * k->C - 2 * hx;
-    const int strips = div_up(k->W, wo);
+    return div_up(W, 32 * k->C - 2 * hx);
+}
+int balanced_segments(const ts_b200_kernel *k, int W, int H, int blocks_per_sm, int warps) {
     const long rw = (long)blocks_per_sm * k->num_sms * warps;
-    const int per_strip = (int)std::max(1L, rw / std::max(1, strips));
-    const int seg = std::max(8, div_up(k->H, per_strip));
+    const int per_strip = (int)std::max(1L, rw / std::max(1, walk_strips(k, W)));
+    const int seg = std::max(8, div_up(H, per_strip));
     return use_walk2(k) ? (seg + 1) & ~1 : seg;
 }
 
@@ -699,23 +700,40 @@ int balanced_segments(const ts_b200_kernel *k, int blocks_per_sm, int warps) {
 // warp means segments of hundreds of rows, which ran 1.3-1.6x slower than
 // 64-128-row segments taken by the persistent warps in turn (8192^2 rotating
 // frame: 2.02 -> 1.35 ms per step in double, 1.72 -> 1.07 in float).
+// A grid wider than its warps (50000 columns are 893 strips) puts more blocks on
+// an SM than asked for, so a row costs what the blocks on the fullest SM make it
+// (50000 x 110 double 62.0 -> 53.8 us, float imaginary time 43.2 -> 35.9).
 constexpr int kMaxAutoSegment = 128;
-void auto_segments(ts_b200_kernel *k) {
-    static const double cost[2][4] = {{1.0, 1.32, 1.70, 2.13}, {1.0, 1.09, 1.42, 2.30}};
-    const int bps = std::min(4, std::max(1, k->resident_blocks / std::max(1, k->num_sms)));
-    const bool walk2 = use_walk2(k);
-    double best = 0.0;
-    k->seg_h = kMaxAutoSegment;
-    for (int b = bps; b >= 1; --b) {
-        const int seg = balanced_segments(k, b, k->warps);
+
+// Rows per segment of a W x H tile with at most `most` blocks per SM and their
+// cost (walked rows times a row's cost, in rows of one block per SM).
+struct WalkShape {
+    int seg;
+    double cost;
+};
+WalkShape walk_shape(const ts_b200_kernel *k, int W, int H, int most) {
+    static const double row_cost[2][4] = {{1.0, 1.32, 1.70, 2.13}, {1.0, 1.09, 1.42, 2.30}};
+    auto cost = [&](int seg) {
+        const long tasks = (long)walk_strips(k, W) * div_up(H, seg);
+        const int per_sm = div_up(tasks, k->warps * k->num_sms);  // blocks on the fullest SM
+        return (std::min(seg, H) + 2 * (k->rot ? 6 : 4)) * row_cost[k->rot][std::min(per_sm, most) - 1] *
+               div_up(per_sm, most);
+    };
+    WalkShape best{kMaxAutoSegment, 0.0};
+    for (int b = most; b >= 1; --b) {
+        const int seg = balanced_segments(k, W, H, b, k->warps);
         // the checked walk keeps the most blocks
-        if (seg > kMaxAutoSegment || (b < bps && !walk2)) break;
-        const double c = (seg + 2 * (k->rot ? 6 : 4)) * cost[k->rot][b - 1];
-        if (b == bps || c < best) {
-            best = c;
-            k->seg_h = seg;
-        }
+        if (seg > kMaxAutoSegment || (b < most && !use_walk2(k))) break;
+        const double c = cost(seg);
+        if (b == most || c < best.cost) best = WalkShape{seg, c};
     }
+    if (best.cost == 0.0) best.cost = cost(best.seg);
+    return best;
+}
+
+void auto_segments(ts_b200_kernel *k) {
+    const int most = std::min(4, std::max(1, k->resident_blocks / std::max(1, k->num_sms)));
+    k->seg_h = walk_shape(k, k->W, k->H, most).seg;
 }
 
 // Programmatic dependent launch of a row walk's steps: where it was asked for
@@ -732,9 +750,7 @@ bool walk_pdl(const ts_b200_kernel *k) {
 // part: the launch covers the part's row windows (no padding).
 void geometry(const ts_b200_kernel *k, int *strips, int *segs, int *blocks, size_t *smem,
               bool pad = true, const tsbh::StepPart *part = nullptr) {
-    const int hx = (k->rot || k->cyl) ? 8 : 4;  // Variant::HX
-    const int wo = 32 * k->C - 2 * hx;
-    *strips = div_up(k->W, wo);
+    *strips = walk_strips(k, k->W);
     const int sh = eff_seg(k);
     if (part && part->a1 > 0) {
         *segs = div_up(part->a1 - part->a0, sh) +
@@ -2137,7 +2153,7 @@ int ts_b200_autotune(ts_b200_kernel *k, int trial_steps) {
         // balanced shapes (one task per warp at b blocks per SM) and short
         // segments taken by the persistent warps in turn
         int cand[24], nc = 0;
-        for (int b = 1; b <= bps && nc < 20; ++b) cand[nc++] = balanced_segments(k, b, warps);
+        for (int b = 1; b <= bps && nc < 20; ++b) cand[nc++] = balanced_segments(k, k->W, k->H, b, warps);
         for (int sh : {32, 64, 128})
             if (sh < k->H) cand[nc++] = sh;
         for (int c = 0; c < nc && st == TS_B200_OK; ++c) {
