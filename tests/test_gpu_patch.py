@@ -301,3 +301,36 @@ def test_asking_for_a_walk_or_overlap_after_steps_keeps_the_evolution():
             k.step(False)
             res.append(k.get_state())
     assert np.array_equal(res[0], res[1])
+
+
+# tiles of few rows and many columns: patches while their regions are resident at
+# once or few beside what a walk would take, else the walk
+@pytest.mark.parametrize("N,Ny,imag,precision,cyl,walk", [
+    (50000, 1, False, 0, False, 2), (50000, 9, False, 0, False, 2), (50000, 3, True, 1, False, 2),
+    (24000, 1, True, 0, False, 2), (50000, 9, False, 1, True, 2), (5000, 9, False, 0, False, 3),
+    (11000, 24, True, 0, False, 3), (1, 20000, False, 0, False, 3)])
+def test_wide_tiles_of_few_rows_are_walked(N, Ny, imag, precision, cyl, walk):
+    from trottersuzuki_b200 import Kernel
+    if cyl:
+        lat = O.Lattice(N, 0.2 * N, Ny, 0.2 * Ny, False, False, cylindrical=True)
+    else:
+        lat = O.Lattice(N, 0.2 * N, Ny, 0.2 * Ny)
+    rng = np.random.default_rng(2)
+    psi0 = 0.1 * (rng.standard_normal(lat.shape) + 1j * rng.standard_normal(lat.shape))
+    V = rng.uniform(0.0, 2.0, lat.shape)
+    n0 = O.expectations(lat, psi0)["norm2"] if imag else 0.0
+    p = lat.params(1e-3, imag, 1.0, 2.0, 0.0, norm0=n0)
+    out = []
+    for checked in (False, True):
+        with Kernel(desc_from_params(p, precision)) as k:
+            if checked:
+                k.set_walk(0)
+            k.set_state(psi0)
+            k.set_exp_potential(*O.exp_table(V, 1e-3, imag))
+            k.evolve(5)
+            assert k.launch_shape()["walk"] == (0 if checked else walk)
+            out.append(k.get_state())
+    if imag and precision:
+        assert np.abs(out[0] - out[1]).max() <= 5 * 2.0 ** -23 * np.abs(out[1]).max()
+    else:
+        _close(*out, imag)

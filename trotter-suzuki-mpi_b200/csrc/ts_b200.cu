@@ -902,6 +902,26 @@ int patch_regions(const ts_b200_kernel *k, int n, int *nx, int *ny) {
 //   float, 4 halo columns: 512^2 6.5 / 8.1 / 9.2, 768^2 9.1 / 10.1 / 10.5,
 //     1024^2 13.3 / 11.9 / 13.1, 1280^2 - / 16.2 / 15.0 (imaginary time 1536^2
 //     - / 17.8 / 18.2)
+// On a tile of few rows and many columns a walk has little to walk (9 rows per
+// strip of a single row), while its regions are as many as those of a square: the
+// walk takes it where its cost (walk_shape) falls short of that of the limit's
+// square by more than the regions do (and by 15 %, so that the limits of ordinary
+// tiles stay); regions that are resident at once keep their lead.  us per step,
+// patches / walk: 50000 x 1 double 16.8 / 8.1, float imaginary time 15.5 / 7.8, 50000
+// x 24 17.1 / 15.1, float cylinder 50000 x 9 28.7 / 11.0; a cylinder's edge regions
+// check every radial coefficient's bounds (50000 x 50 32.0 / 26.1).
+bool patch_fits(const ts_b200_kernel *k, int n, int most) {
+    int nx, ny;
+    const int regions = patch_regions(k, n, &nx, &ny);
+    if (regions > most) return false;
+    if (k->H >= k->W || regions <= tsb::patch_blocks(n, k->fp32) * k->num_sms) return true;
+    const int hx = (k->rot || k->cyl) ? 8 : 4, hy = k->rot ? 6 : 4;  // Variant::HX, HY
+    const int side = (int)sqrt((double)most * tsb::patch_out(n, hx) * tsb::patch_out(n, hy));
+    const double margin = k->cyl && ny <= 2 ? 1.1 : 0.85;
+    return margin * regions * walk_shape(k, side, side, 4).cost <=
+           most * walk_shape(k, k->W, k->H, 4).cost;
+}
+
 int patch_cells(const ts_b200_kernel *k) {
     if (!k->patch || k->walk2 != 2) return 0;
     int most2, most4 = 0;  // regions
@@ -920,9 +940,8 @@ int patch_cells(const ts_b200_kernel *k) {
         most2 = (k->imag || k->phase == 0) ? 1600 : 2100;
     }
     int nx, ny;
-    if (patch_regions(k, 2, &nx, &ny) <= most2) return 2;
-    if (patch_regions(k, 4, &nx, &ny) <= most4) return 4;
-    return 0;
+    if (patch_regions(k, 2, &nx, &ny) <= most2) return patch_fits(k, 2, most2) ? 2 : 0;
+    return patch_fits(k, 4, most4) ? 4 : 0;
 }
 
 // Grid of the patch step: the regions, taken in turn by the blocks that the
