@@ -334,3 +334,29 @@ def test_wide_tiles_of_few_rows_are_walked(N, Ny, imag, precision, cyl, walk):
         assert np.abs(out[0] - out[1]).max() <= 5 * 2.0 ** -23 * np.abs(out[1]).max()
     else:
         _close(*out, imag)
+
+
+@pytest.mark.parametrize("N,Ny,every,imag", [(32000, 1, 0, False), (44000, 3, 4, False),
+                                             (44000, 1, 4, True), (16000, 9, 0, False)])
+def test_adjoint_of_wide_tiles_of_few_rows(N, Ny, every, imag):
+    """The pass on its default (the walk beyond the resident regions where that has
+    less to do) and on the walk asked for."""
+    import torch
+    from trottersuzuki_b200.adjoint import AdjointEngine
+    lat = O.Lattice(N, 0.2 * N, Ny, 0.2 * Ny)
+    rng = np.random.default_rng(4)
+    psi0 = 0.1 * (rng.standard_normal(lat.shape) + 1j * rng.standard_normal(lat.shape))
+    n0 = O.expectations(lat, psi0)["norm2"] if imag else 0.0
+    p = lat.params(1e-3, imag, 1.0, 8.0 if every else 0.0, norm0=n0)
+    v = torch.tensor(rng.uniform(0.0, 2.0, lat.shape), device="cuda")
+    psi = torch.tensor(psi0, device="cuda")
+    out = []
+    for rows in (0, 6):
+        e = AdjointEngine(desc_from_params(p), 1e-3, 10, every)
+        if rows:
+            e.set_segments(adjoint_rows=rows)
+        e.forward(v, psi)
+        out.append([t.cpu().numpy() for t in e.backward(psi)])
+        e.close()
+    for got, old in zip(*out):
+        _close(got, old, imag)

@@ -246,10 +246,34 @@ cudaError_t launch_adj(ts_b200_adjoint *a, int mode, int phase, const AdjArgs &a
 // 900^2 23.5 / 28.9, 1024^2 34.4 / 32.0; checkpointed GPE 512^2 13.3 / 32.6,
 // 1024^2 44.3 / 54.4, 1280^2 80.5 / 74.4; imaginary time 512^2 18.7 / 33.6,
 // 1024^2 49.1 / 52.7, 1280^2 73.8 / 64.2).
+// On a tile of few rows and many columns the walk has little to walk: it takes it
+// where its cost falls short of that of the limit's square by more than the
+// regions do, as in patch_fits (ts_b200.cu; a row costs half as much again once the
+// warps pass half of those resident; margins by the measured crossings).  Linear 32000
+// x 1 16.7 / 10.3, checkpointed 44000 x 1 28.8 / 18.9, 44000 x 9 39.6 / 33.7.
+int adj_segment_rows(const ts_b200_adjoint *a, int W, int H) {
+    const int strips = div_up(W, AdjVariant<0, 0>::WO);
+    const int per_strip = std::max(1, a->blocks * a->warps / strips);
+    const int rows = std::max(a->imag ? 6 : 4, div_up(H, per_strip));
+    return rows + (rows & 1);
+}
+double adj_walk_cost(const ts_b200_adjoint *a, int W, int H) {
+    const int rows = adj_segment_rows(a, W, H), warps = std::max(1, a->blocks * a->warps);
+    const long tasks = (long)div_up(W, AdjVariant<0, 0>::WO) * div_up(H, rows);
+    return (std::min(rows, H) + 8) * (2 * tasks > warps ? 1.5 : 1.0) * div_up(tasks, warps);
+}
 int adj_patch_regions(const ts_b200_adjoint *a) {
     constexpr int out = tsb::patch_out(tsb::kAdjPatch, AdjVariant<0, 0>::HX);
     const long n = (long)div_up(a->W, out) * div_up(a->H, out);
-    return a->patch && n <= (a->every > 0 ? 1900 : 1500) ? (int)n : 0;
+    const int most = a->every > 0 ? 1900 : 1500;
+    if (!a->patch || n > most) return 0;
+    if (a->H < a->W && n > tsb::kAdjPatchBlocks * a->k->num_sms) {
+        const int side = (int)std::sqrt((double)most) * out;
+        if ((a->imag ? 0.7 : 0.85) * n * adj_walk_cost(a, side, side) >
+            most * adj_walk_cost(a, a->W, a->H))
+            return 0;
+    }
+    return (int)n;
 }
 
 // One pass with the arguments of its fields.
@@ -541,10 +565,7 @@ int ts_b200_adjoint_create(const ts_b200_desc *d, double delta_t, int steps, int
         // 512^2 the pass took 63.6 / 128.3 / 162.8 ms (linear, checkpointed,
         // imaginary time, 3000 steps) at 4 / 4 / 6 rows against 67.2 /
         // 144.3 / 169.0 at 8 and 89 / 195 / 235 at 2
-        const int strips = div_up(a->W, AdjVariant<0, 0>::WO);
-        const int per_strip = std::max(1, a->blocks * a->warps / strips);
-        a->seg_h = std::max(a->imag ? 6 : 4, div_up(a->H, per_strip));
-        a->seg_h += a->seg_h & 1;
+        a->seg_h = adj_segment_rows(a, a->W, a->H);
         // block partials of the reductions (adjoint steps and the dot kernel)
         if (a->imag) alloc(reinterpret_cast<void **>(&a->partials),
                            sizeof(double) * std::max(a->blocks, 1024));
