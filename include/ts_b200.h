@@ -181,7 +181,10 @@ int ts_b200_squared_norm_noalloc(const void *psi, int precision, size_t pitch, i
 /* Device-resident access (for callers that already hold device memory, such
  * as a torch binding or a benchmark).  `aos` is a device array of dim_y rows
  * of dim_x interleaved complex numbers in the kernel's precision with row
- * pitch `pitch` cells. */
+ * pitch `pitch` cells.  A kernel copies rows of the handle's own GPU; the two
+ * setters leave memory that it does not own (another GPU's, host memory) to the
+ * runtime's copy.  ts_b200_get_state_device writes from a kernel: to memory that
+ * the handle's GPU can write. */
 int ts_b200_set_state_device(ts_b200_kernel *k, const void *aos, size_t pitch);
 int ts_b200_get_state_device(ts_b200_kernel *k, void *aos, size_t pitch);
 int ts_b200_set_exp_potential_device(ts_b200_kernel *k, const void *table, size_t pitch);

@@ -360,3 +360,61 @@ def test_adjoint_of_wide_tiles_of_few_rows(N, Ny, every, imag):
         e.close()
     for got, old in zip(*out):
         _close(got, old, imag)
+
+
+@pytest.mark.parametrize("precision,imag", [(0, False), (1, True)])
+def test_states_and_tables_not_of_this_gpu_are_copied_by_the_runtime(precision, imag):
+    """Rows in pinned host memory stand for all memory that the handle's GPU does not
+    own: no kernel reads them."""
+    import torch
+    from trottersuzuki_b200 import Kernel
+    from trottersuzuki_b200.kernel import launch_count
+    lat, psi0, V = seeded_case(45, 10.0, 31)
+    p = lat.params(1e-3, imag, 1.0, 1.0, 0.0, norm0=1.0 if imag else 0.0)
+    ctype = torch.complex64 if precision else torch.complex128
+    src = torch.tensor(psi0).to(ctype)
+    tab = torch.tensor(np.exp((-1e-3 if imag else -1e-3j) * V))
+    tab = tab.to(torch.float32 if precision else torch.float64) if imag else tab.to(ctype)
+    out = []
+    for place in (lambda t: t.pin_memory(), lambda t: t.cuda()):
+        with Kernel(desc_from_params(p, precision=precision)) as k:
+            s, t = place(src), place(tab)
+            before = launch_count()
+            k.set_state_device(s.data_ptr(), lat.dim_x)
+            k.set_exp_potential_device(t.data_ptr(), lat.dim_x)
+            out.append(launch_count() - before)
+            k.step(exchange=False)
+            out.append(k.get_state())
+    assert (out[0], out[2]) == (0, 2)
+    assert np.array_equal(out[1], out[3])
+
+
+def test_device_states_and_tables_under_capture():
+    """A stream capture takes the setters, a step and the state's copy."""
+    import torch
+    from trottersuzuki_b200 import Kernel
+    lat, psi0, V = seeded_case(45, 10.0, 31)
+    p = lat.params(1e-3, False, 1.0, 1.0)
+    src = torch.tensor(psi0, device="cuda")
+    tab = torch.tensor(np.exp(-1e-3j * V), device="cuda")
+    out = torch.zeros_like(src)
+    with Kernel(desc_from_params(p)) as k:
+        def program():
+            k.set_state_device(src.data_ptr(), lat.dim_x)
+            k.set_exp_potential_device(tab.data_ptr(), lat.dim_x)
+            k.evolve(3)
+            k.get_state_device(out.data_ptr(), lat.dim_x)
+        stream = torch.cuda.Stream()
+        k.set_stream(stream.cuda_stream)
+        with torch.cuda.stream(stream):
+            program()
+            torch.cuda.synchronize()
+            ref = out.clone()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                program()
+            out.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+        k.set_stream(0)

@@ -1411,12 +1411,25 @@ int upload_kinetic_schedule(ts_b200_kernel *k) {
 
 int grid_for(size_t n) { return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 8192)); }
 
+// Whether a kernel of the handle may read `p`: the handle's GPU owns it.  What it
+// does not own (another GPU's memory, with or without peer access, host memory)
+// is the runtime's to copy or to refuse: a kernel would fault on part of it.
+bool own_memory(const ts_b200_kernel *k, const void *p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == k->device;
+}
+
 // Rows of W elements of `cell` bytes (4, 8 or 16), pitches in elements, on the
-// handle's stream; what is not aligned to an element goes through the runtime.
+// handle's stream; by_kernel: both are the handle's GPU's memory.  Else, and what
+// is not aligned to an element, goes through the runtime.
 int copy_rows(ts_b200_kernel *k, void *dst, size_t dpitch, const void *src, size_t spitch,
-              size_t cell, Scalars *reset) {
+              size_t cell, Scalars *reset, bool by_kernel) {
     const dim3 grid = copy_grid(k->W, k->H);
-    if (((uintptr_t)dst | (uintptr_t)src) % cell != 0) {
+    if (!by_kernel || ((uintptr_t)dst | (uintptr_t)src) % cell != 0) {
         TSB_CHECK(k, cudaMemcpy2DAsync(dst, dpitch * cell, src, spitch * cell, k->W * cell, k->H,
                                        cudaMemcpyDeviceToDevice, k->stream));
         const double one = 1.0;
@@ -1697,12 +1710,13 @@ int ts_b200_set_exp_potential(ts_b200_kernel *k, const double *re, const double 
 
 int ts_b200_set_state_device(ts_b200_kernel *k, const void *aos, size_t pitch) {
     if (!k || !aos || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    return copy_rows(k, k->psi[k->cur], k->P, aos, pitch, k->cell, k->scal);
+    return copy_rows(k, k->psi[k->cur], k->P, aos, pitch, k->cell, k->scal, own_memory(k, aos));
 }
 
 int ts_b200_get_state_device(ts_b200_kernel *k, void *aos, size_t pitch) {
     if (!k || !aos || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    if (!k->imag) return copy_rows(k, aos, pitch, k->psi[k->cur], k->P, k->cell, nullptr);
+    if (!k->imag)
+        return copy_rows(k, aos, pitch, k->psi[k->cur], k->P, k->cell, nullptr, true);
     const dim3 grid = copy_grid(k->W, k->H);
     if (k->fp32)
         scale_rows_kernel<float><<<grid, kCopyThreads, 0, k->stream>>>(
@@ -1719,7 +1733,7 @@ int ts_b200_get_state_device(ts_b200_kernel *k, void *aos, size_t pitch) {
 
 int ts_b200_set_exp_potential_device(ts_b200_kernel *k, const void *table, size_t pitch) {
     if (!k || !table || pitch < (size_t)k->W) return TS_B200_INVALID_ARGUMENT;
-    return copy_rows(k, k->tab, k->P, table, pitch, k->tab_cell, nullptr);
+    return copy_rows(k, k->tab, k->P, table, pitch, k->tab_cell, nullptr, own_memory(k, table));
 }
 
 int ts_b200_set_potential_device(ts_b200_kernel *k, const double *potential, size_t pitch,
