@@ -316,16 +316,17 @@ int ts_b200_stream_wait(ts_b200_kernel *k, void *stream);
 int ts_b200_stream_signal(ts_b200_kernel *k, void *stream);
 int ts_b200_synchronize(ts_b200_kernel *k);
 
-/* Geometry of the fused step launch chosen for this tile (for reporting):
- * cells per lane, rows per segment, warps per block, ring depth, tasks, and
- * the row walk (0 checked; 1 or 2: look-ahead, rows per iteration).  walk 3:
- * register patches; then cells_per_lane is the side of a thread's patch,
- * strips x segments the regions, segment_rows the rows that one writes. */
+/* Geometry of the launches of ts_b200_evolve chosen for this tile (for reporting;
+ * of ts_b200_step too where steps is 1): cells per lane, rows per segment, warps per
+ * block, ring depth, tasks, the row walk (0 checked; 1 or 2: look-ahead, rows per
+ * iteration) and the steps that a launch takes.  walk 3: register patches; then
+ * cells_per_lane is the side of a thread's patch, strips x segments the regions,
+ * segment_rows the rows that one writes. */
 typedef struct {
     int32_t cells_per_lane, segment_rows, warps_per_block, ring_depth;
     int32_t strips, segments, blocks, threads;
     int64_t smem_bytes;
-    int32_t walk, reserved;
+    int32_t walk, steps;
 } ts_b200_launch_shape;
 
 int ts_b200_launch_info(const ts_b200_kernel *k, ts_b200_launch_shape *out);

@@ -418,3 +418,27 @@ def test_device_states_and_tables_under_capture():
             torch.cuda.synchronize()
         assert torch.equal(out, ref)
         k.set_stream(0)
+
+
+# side of the patches, steps per launch, rows written by a region
+@pytest.mark.parametrize("N,per,imag,precision,side,steps,rows", [
+    (64, False, False, 0, 2, 3, 8), (200, False, False, 0, 2, 2, 16), (700, False, False, 0, 4, 2, 48),
+    (1200, False, False, 1, 4, 2, 48), (64, True, False, 0, 2, 1, 24), (64, False, True, 0, 2, 1, 24)])
+def test_launch_shape_tells_what_evolve_launches(N, per, imag, precision, side, steps, rows):
+    from trottersuzuki_b200 import Kernel
+    from trottersuzuki_b200.kernel import launch_count
+    lat, psi0, V = seeded_case(N, 10.0, None, (per, per))
+    p = lat.params(1e-4, imag, 1.0, 1.0, 0.0, norm0=1.0 if imag else 0.0)
+    with Kernel(desc_from_params(p, precision)) as k:
+        k.set_state(psi0)
+        k.set_exp_potential(*O.exp_table(V, 1e-4, imag))
+        shape = k.launch_shape()
+        assert (shape["walk"], shape["cells_per_lane"]) == (3, side)
+        assert (shape["steps"], shape["segment_rows"]) == (steps, rows)
+        across = -(-lat.dim_x // rows)
+        assert (shape["strips"], shape["segments"]) == (across, -(-lat.dim_y // rows))
+        before = launch_count()
+        k.evolve(6)
+        assert launch_count() - before == 6 // steps
+        k.set_walk(2)
+        assert (k.launch_shape()["walk"], k.launch_shape()["steps"]) == (2, 1)

@@ -712,7 +712,7 @@ int ts_b200_batch_launch_info(ts_b200_batch *b, ts_b200_launch_shape *out) {
     out->threads = 32 * b->shape.warps;
     out->smem_bytes = (int64_t)batch_smem(b, b->shape.warps);
     out->walk = b->walk;
-    out->reserved = 0;
+    out->steps = 1;
     return TS_B200_OK;
 }
 

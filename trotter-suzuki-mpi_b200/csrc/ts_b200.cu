@@ -1111,6 +1111,11 @@ Fused fused_steps(const ts_b200_kernel *k) {
     return f;
 }
 
+// Blocks that the GPU holds of them.
+int fused_most(const ts_b200_kernel *k, const Fused &f) {
+    return tsb::patch_steps_blocks(f.n, k->fp32) * k->num_sms;
+}
+
 // f.m steps from buffer `in` to buffer `out` (no buffer flip).
 template <typename T>
 int launch_fused_buffers_t(ts_b200_kernel *k, const Fused &f, const void *in, void *out) {
@@ -1120,8 +1125,7 @@ int launch_fused_buffers_t(ts_b200_kernel *k, const Fused &f, const void *in, vo
     tsbh::fill_step_constants(k, a);
     a.n_strips = f.nx;
     a.n_segs = f.ny;
-    const int most = tsb::patch_steps_blocks(f.n, k->fp32) * k->num_sms;
-    const int blocks = std::min(f.nx * f.ny, most);
+    const int most = fused_most(k, f), blocks = std::min(f.nx * f.ny, most);
     // as step_pdl: not where the next launch's blocks would crowd some of the SMs
     // (us per step without / with, double GPE: 96^2 in 144 blocks of at most 296
     // 1.73 / 2.13, 256^2 in 256 2.89 / 2.55; 4 x 4 patches 512^2 in 121 6.2 / 7.9,
@@ -2036,12 +2040,21 @@ int ts_b200_launch_info(const ts_b200_kernel *k, ts_b200_launch_shape *out) {
     int strips, segs, blocks;
     size_t smem;
     geometry(k, &strips, &segs, &blocks, &smem);
-    if (const int n = patch_cells(k)) {
-        patch_geometry(k, n, &strips, &segs, &blocks);
+    const Fused f = fused_steps(k);
+    const int n = f.m > 1 ? f.n : patch_cells(k);
+    *out = ts_b200_launch_shape{};
+    out->steps = f.m;
+    if (n) {
+        if (f.m > 1) {
+            strips = f.nx;
+            segs = f.ny;
+            blocks = std::min(f.nx * f.ny, fused_most(k, f));
+        } else {
+            patch_geometry(k, n, &strips, &segs, &blocks);
+        }
         const bool all_rows = k->rot || k->cyl;
-        *out = ts_b200_launch_shape{};
         out->cells_per_lane = n;
-        out->segment_rows = tsb::patch_out(n, k->rot ? 6 : 4);
+        out->segment_rows = tsb::patch_out(n, f.m * (k->rot ? 6 : 4));
         out->warps_per_block = 8;
         out->strips = strips;
         out->segments = segs;

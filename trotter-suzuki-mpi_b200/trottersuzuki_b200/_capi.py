@@ -66,7 +66,7 @@ class LaunchShape(C.Structure):
         ("warps_per_block", C.c_int32), ("ring_depth", C.c_int32),
         ("strips", C.c_int32), ("segments", C.c_int32), ("blocks", C.c_int32),
         ("threads", C.c_int32), ("smem_bytes", C.c_int64),
-        ("walk", C.c_int32), ("reserved", C.c_int32),
+        ("walk", C.c_int32), ("steps", C.c_int32),
     ]
 
 
