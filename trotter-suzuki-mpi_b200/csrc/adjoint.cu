@@ -241,11 +241,11 @@ cudaError_t launch_adj(ts_b200_adjoint *a, int mode, int phase, const AdjArgs &a
 }
 
 // Regions of the pass on register patches, 0 where the row walk takes it: on
-// large tiles, and where its segments were asked for (us per step of the
-// reverse pass, patches / walk; linear 256^2 4.8 / 18.5, 512^2 10.5 / 21.3,
-// 900^2 23.5 / 28.9, 1024^2 34.4 / 32.0; checkpointed GPE 512^2 13.3 / 32.6,
-// 1024^2 44.3 / 54.4, 1280^2 80.5 / 74.4; imaginary time 512^2 18.7 / 33.6,
-// 1024^2 49.1 / 52.7, 1280^2 73.8 / 64.2).
+// large tiles (more regions per SM than measured on 148), and where its segments
+// were asked for (us per step of the reverse pass, patches / walk; linear 256^2
+// 4.8 / 18.5, 512^2 10.5 / 21.3, 900^2 23.5 / 28.9, 1024^2 34.4 / 32.0;
+// checkpointed GPE 512^2 13.3 / 32.6, 1024^2 44.3 / 54.4, 1280^2 80.5 / 74.4;
+// imaginary time 512^2 18.7 / 33.6, 1024^2 49.1 / 52.7, 1280^2 73.8 / 64.2).
 // On a tile of few rows and many columns the walk has little to walk: it takes it
 // where its cost falls short of that of the limit's square by more than the
 // regions do, as in patch_fits (ts_b200.cu; a row costs half as much again once the
@@ -265,7 +265,7 @@ double adj_walk_cost(const ts_b200_adjoint *a, int W, int H) {
 int adj_patch_regions(const ts_b200_adjoint *a) {
     constexpr int out = tsb::patch_out(tsb::kAdjPatch, AdjVariant<0, 0>::HX);
     const long n = (long)div_up(a->W, out) * div_up(a->H, out);
-    const int most = a->every > 0 ? 1900 : 1500;
+    const int most = (a->every > 0 ? 1900 : 1500) * a->k->num_sms / 148;
     if (!a->patch || n > most) return 0;
     if (a->H < a->W && n > tsb::kAdjPatchBlocks * a->k->num_sms) {
         const int side = (int)std::sqrt((double)most) * out;

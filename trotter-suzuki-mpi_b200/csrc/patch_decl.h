@@ -18,6 +18,27 @@ constexpr int patch_steps_blocks(int n, bool fp32) { return fp32 && n == 2 ? 4 :
 // a halo of h cells per sweep direction (whole patches).
 constexpr int patch_out(int n, int h) { return 16 * n - 2 * ((h + n - 1) / n * n); }
 
+// Regions up to which patches of 2 x 2 cells, and past those of 4 x 4 (0: never),
+// take a tile's step on a GPU of `sms` SMs; pair: one species of two.  The limits
+// were measured on 148 SMs (patch_cells in ts_b200.cu): places and turns of the
+// regions go by the SMs.
+struct PatchLimits {
+    int side2, side4;
+};
+constexpr PatchLimits patch_limits(bool fp32, bool imag, bool rot, bool cyl, bool pair, bool phase,
+                                   int sms) {
+    const PatchLimits m = pair   ? PatchLimits{fp32 ? 520 : 750, 0}
+                          : rot  ? PatchLimits{320, fp32 ? 2000 : 870}
+                          : cyl  ? PatchLimits{260, fp32 ? 1100 : 300}
+                          : fp32 ? PatchLimits{1100, imag ? 900 : 430}
+                                 : PatchLimits{imag || !phase ? 1600 : 2100, 0};
+    return PatchLimits{m.side2 * sms / 148, m.side4 * sms / 148};
+}
+static_assert(patch_limits(false, false, false, false, false, true, 148).side2 == 2100 &&
+                  patch_limits(false, false, false, false, false, true, 74).side2 == 1050 &&
+                  patch_limits(true, false, true, false, false, true, 74).side4 == 1000,
+              "half the SMs, half the regions");
+
 // n: cells of a thread's patch per side (2 or 4); phase as for the row walks
 // (| 16: potential rows); pdl: programmatic dependent launch.
 cudaError_t launch_patch_f64_real(int n, bool rot, int phase, const StepArgs<double> &a,

@@ -880,28 +880,7 @@ int patch_regions(const ts_b200_kernel *k, int n, int *nx, int *ny) {
     return (long)*nx * *ny > INT32_MAX ? INT32_MAX : *nx * *ny;
 }
 
-// Cells per side of a thread's patch in the register-patch step (patch.cuh),
-// 0 where a row walk steps the tile: on large tiles, and where a walk or its
-// shape has been asked for.  Patches of 2 x 2 cells have the shorter latency,
-// of 4 x 4 fewer recomputed cells, the walk the best throughput.  The limits
-// are the region counts up to which each was the fastest of the three on
-// square tiles (us per step, 2 x 2 / 4 x 4 / walk):
-//   double, 4 halo columns: 256^2 3.3 / 8.4 / 9.3, 512^2 6.2 / 8.7 / 10.9,
-//     1024^2 15.0 / 18.8 / 16.9, 1280^2 26.0 / 23.6 / 20; imaginary time
-//     1024^2 17.2 / 19.0 / 16.8, linear 13.7 / - / 12.8; potential rows 18.0 /
-//     28.0 / 20.7
-//   one species of a pair: 640^2 12.8 / - / 14.3, 768^2 17.8 / 21.0 / 15.7;
-//     float 512^2 8.9 / 13.0 / 11.6, 640^2 12.2 / 13.2 / 11.6
-//   rotating frame, double: 256^2 5.9 / 10.1 / 18.8, 512^2 13.3 / 10.6 / 20.6,
-//     1024^2 41.7 / 26.2 / 32.1, 1300^2 - / 41.0 / 42.3
-//   rotating frame, float: 256^2 6.6 / 9.4 / 25.2, 512^2 11.0 / 9.9 / 25.8,
-//     2048^2 96.1 / 48.4 / 54.4, 4096^2 388 / 171 / 152
-//   cylinder, double: 256^2 7.9 / 11.0 / 12.8, 512^2 13.3 / 11.8 / 13.9,
-//     830^2 - / 15.1 / 17.7, 1024^2 32.1 / 26.2 / 21.3
-//   cylinder, float: 512^2 9.8 / 9.1 / 11.4, 1536^2 39.6 / 23.2 / 24.1
-//   float, 4 halo columns: 512^2 6.5 / 8.1 / 9.2, 768^2 9.1 / 10.1 / 10.5,
-//     1024^2 13.3 / 11.9 / 13.1, 1280^2 - / 16.2 / 15.0 (imaginary time 1536^2
-//     - / 17.8 / 18.2)
+// Whether patches of n x n cells take the tile's step, up to `most` regions.
 // On a tile of few rows and many columns a walk has little to walk (9 rows per
 // strip of a single row), while its regions are as many as those of a square: the
 // walk takes it where its cost (walk_shape) falls short of that of the limit's
@@ -922,26 +901,35 @@ bool patch_fits(const ts_b200_kernel *k, int n, int most) {
            most * walk_shape(k, k->W, k->H, 4).cost;
 }
 
+// Cells per side of a thread's patch in the register-patch step (patch.cuh),
+// 0 where a row walk steps the tile: on large tiles, and where a walk or its
+// shape has been asked for.  Patches of 2 x 2 cells have the shorter latency,
+// of 4 x 4 fewer recomputed cells, the walk the best throughput.  The limits
+// (tsb::patch_limits) are the region counts up to which each was the fastest of the
+// three on square tiles (us per step, 2 x 2 / 4 x 4 / walk):
+//   double, 4 halo columns: 256^2 3.3 / 8.4 / 9.3, 512^2 6.2 / 8.7 / 10.9,
+//     1024^2 15.0 / 18.8 / 16.9, 1280^2 26.0 / 23.6 / 20; imaginary time
+//     1024^2 17.2 / 19.0 / 16.8, linear 13.7 / - / 12.8; potential rows 18.0 /
+//     28.0 / 20.7
+//   one species of a pair: 640^2 12.8 / - / 14.3, 768^2 17.8 / 21.0 / 15.7;
+//     float 512^2 8.9 / 13.0 / 11.6, 640^2 12.2 / 13.2 / 11.6
+//   rotating frame, double: 256^2 5.9 / 10.1 / 18.8, 512^2 13.3 / 10.6 / 20.6,
+//     1024^2 41.7 / 26.2 / 32.1, 1300^2 - / 41.0 / 42.3
+//   rotating frame, float: 256^2 6.6 / 9.4 / 25.2, 512^2 11.0 / 9.9 / 25.8,
+//     2048^2 96.1 / 48.4 / 54.4, 4096^2 388 / 171 / 152
+//   cylinder, double: 256^2 7.9 / 11.0 / 12.8, 512^2 13.3 / 11.8 / 13.9,
+//     830^2 - / 15.1 / 17.7, 1024^2 32.1 / 26.2 / 21.3
+//   cylinder, float: 512^2 9.8 / 9.1 / 11.4, 1536^2 39.6 / 23.2 / 24.1
+//   float, 4 halo columns: 512^2 6.5 / 8.1 / 9.2, 768^2 9.1 / 10.1 / 10.5,
+//     1024^2 13.3 / 11.9 / 13.1, 1280^2 - / 16.2 / 15.0 (imaginary time 1536^2
+//     - / 17.8 / 18.2)
 int patch_cells(const ts_b200_kernel *k) {
     if (!k->patch || k->walk2 != 2) return 0;
-    int most2, most4 = 0;  // regions
-    if ((k->phase & 3) == 3) {
-        most2 = k->fp32 ? 520 : 750;
-    } else if (k->rot) {
-        most2 = 320;
-        most4 = k->fp32 ? 2000 : 870;
-    } else if (k->cyl) {
-        most2 = 260;
-        most4 = k->fp32 ? 1100 : 300;
-    } else if (k->fp32) {
-        most2 = 1100;
-        most4 = k->imag ? 900 : 430;
-    } else {
-        most2 = (k->imag || k->phase == 0) ? 1600 : 2100;
-    }
+    const tsb::PatchLimits most = tsb::patch_limits(k->fp32, k->imag, k->rot, k->cyl,
+                                                    (k->phase & 3) == 3, k->phase != 0, k->num_sms);
     int nx, ny;
-    if (patch_regions(k, 2, &nx, &ny) <= most2) return patch_fits(k, 2, most2) ? 2 : 0;
-    return patch_fits(k, 4, most4) ? 4 : 0;
+    if (patch_regions(k, 2, &nx, &ny) <= most.side2) return patch_fits(k, 2, most.side2) ? 2 : 0;
+    return patch_fits(k, 4, most.side4) ? 4 : 0;
 }
 
 // Grid of the patch step: the regions, taken in turn by the blocks that the
