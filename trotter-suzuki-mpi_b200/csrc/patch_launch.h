@@ -26,7 +26,9 @@ cudaError_t launch_patch_variant(int n, const StepArgs<T> &a, int blocks, cudaSt
                                  bool pdl) {
     using V = Variant<T, 2, IMAG, ROT, PHASE>;
     if (n == 2) return launch_patch_shape<PatchShape<V, 2>>(a, blocks, st, pdl);
-    if (n == 4) return launch_patch_shape<PatchShape<V, 4>>(a, blocks, st, pdl);
+    // only where patch_cells can choose them
+    if constexpr (patch_limits(sizeof(T) == 4, IMAG, ROT, V::CYL, V::PB, V::PHASE, 148).side4 > 0)
+        if (n == 4) return launch_patch_shape<PatchShape<V, 4>>(a, blocks, st, pdl);
     return cudaErrorInvalidValue;
 }
 
