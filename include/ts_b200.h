@@ -337,7 +337,9 @@ int ts_b200_set_launch(ts_b200_kernel *k, int cells_per_lane, int segment_rows, 
                        int ring_depth);
 
 /* Row walk of the fused step (no counterpart in the reference; every walk
- * performs the same operations per cell).  By default small and middle-sized
+ * performs the same operations per cell, but for nonlinear phases past 2^-8 in
+ * imaginary time and in a double rotating frame, whose evaluation a warp chooses
+ * for all its cells).  By default small and middle-sized
  * tiles are stepped by register patches (a block holds a region of the tile
  * in registers; launch info reports walk 3) and larger ones by walk 2; a call
  * of this or of ts_b200_set_launch chooses a row walk: 2 the look-ahead walk of

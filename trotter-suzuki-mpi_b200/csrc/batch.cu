@@ -181,11 +181,11 @@ size_t batch_smem(const ts_b200_batch *b, int warps) {
 // segment's 8 halo rows, times what a row costs at that many warps are
 // fewest.  Batches that would need segments above kMaxSegment rows take their
 // tasks in turns: in double the shortest segments whose tasks fill the fewest
-// turns, in float kMaxSegment.  us per step with kMaxSegment everywhere -> now
-// (double / float): 8 tiles of 48^2 .. 200^2 61.5 -> 9.9 / 44.3 -> 9.7, 32 of 300^2
-// 61.3 -> 31.3 / 45.6 -> 23.5, 4 of 256^2 .. 1024^2 61.0 -> 20.6 / 44.8 -> 16.4, 32 of
-// 152^2 .. 952^2 98 -> 92 / 67.0 -> 61.7, 20 of 1000^2 194 -> 180 (imaginary time
-// 171 -> 144) / 100 -> 97.
+// turns, in float kMaxSegment.  us per step with kMaxSegment everywhere and plain
+// launches -> now (double / float): 8 tiles of 48^2 .. 200^2 61.5 -> 9.9 / 46.8 -> 8.3,
+// 32 of 300^2 62.0 -> 30.4 / 48.8 -> 22.8, 4 of 256^2 .. 1024^2 61.7 -> 19.9 / 47.2 ->
+// 14.8, 32 of 152^2 .. 952^2 104 -> 91 / 68.5 -> 58.5, 20 of 1000^2 203 -> 178
+// (imaginary time 174 -> 143) / 97.6 -> 93.5.
 constexpr int kMaxSegment = 128, kMinSegment = 8;
 
 int auto_segment(const ts_b200_batch *b) {

@@ -21,7 +21,7 @@
 // and a walk's short segments recompute more (8-row segments 2.3 cells per
 // cell written, a 32 x 32 region 1.8, a 64 x 64 one 1.3).  On large tiles the
 // walk's asynchronous row copies and its 4 independent warps per scheduler
-// keep the FP64 pipe busier (2048^2 double: 48 us against 63).
+// keep the FP64 pipe busier (2048^2 double: 38.6 us against 63).
 //
 // Regions that reach over the tile's edge (EDGE) mask the pairs across it:
 // the identity, as closed boundaries skip them (src/cpucartesian.cpp:4-70);

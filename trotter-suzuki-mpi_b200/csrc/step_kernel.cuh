@@ -520,17 +520,19 @@ __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 // or past the second replace its result.  With two branches instead of three
 // for the whole warp more of the row body is scheduled across them: the 2048^2
 // double real-time step took 38.7 us against 43.9-48.0 (phases of the second
-// tier 46.6 / 49.7, of the library 65.2 / 63.6).
+// tier 46.4 / 46.9, of the library 63.3 / 61.9; 3000^2 81.7 / 109 / 119 us in the
+// three, 93.0 / 105 / 119 before).
 // ROT: all but the first path in a function of its own, for the rotating frame,
 // whose row body is bound by instruction fetch.  Double, against the same tiers
 // in line: 1500^2 50.3 -> 47.8 us, 2048^2 76.6 -> 75.6, 3000^2 139.0 -> 138.8, 4096^2
 // 296.8 -> 293.4; 4096^2 with phases of the second tier 361 -> 375, of the library
-// 398 -> 409.
+// 398 -> 409.  (Before double had branches per cell elsewhere the same step in
+// line took 75.5 us at 2048^2, 139.0 at 3000^2, 289.9 / 355 / 392 at 4096^2.)
 // Float, against two series and the library by the warp's choice (first tier /
-// second / library): 1200^2 12.8 / 13.6 / 22.9 -> 11.6 / 11.8 / 21.8, 2048^2 26.1
-// / 28.0 / 44.2 -> 24.9 / 25.1 / 41.8; rotating frame 4096^2 142.5 / 179.8 / 235
-// -> 143.2 / 177.9 / 216, 8192^2 547 / 652 / 979 -> 549 / 552 / 871 (in line, as
-// elsewhere in float, 565 / 557 / 857).
+// second / library): 1200^2 12.7 / 13.7 / 22.9 -> 11.6 / 11.8 / 21.8, 2048^2 26.3
+// / 28.1 / 44.4 -> 25.0 / 25.1 / 41.9; rotating frame 2300^2 62.3 / 68.9 / 94.4 ->
+// 62.2 / 61.9 / 99.3, 4096^2 145 / 180 / 235 -> 143 / 178 / 216, 8192^2 562 / 657 /
+// 980 -> 563 / 563 / 872 (in line, as elsewhere in float, 3 % more in the first).
 // Returns sin(th) and cos(th) (cos(th) - 1 in delta form).  The comparisons are
 // exact in either precision.
 __device__ __forceinline__ bool phase_tiny(double th) { return fabs(th) < 0.00390625; }

@@ -1070,7 +1070,9 @@ int launch_step_t(ts_b200_kernel *k, int exchange, bool dry = false) {
 //   float, GPE: 64^2 1.98 / 2.49 / - / 4.31, 256^2 - / 3.31 / - / 5.09, 384^2 - /
 //     4.16 / 5.03 / 5.61, 512^2 - / 6.81 / 4.97 / 6.54, 816^2 - / - / 6.45 / 9.79,
 //     1200^2 - / - / 12.8 / 14.1, 1400^2 - / - / 16.5 / 15.8; with Lee-Huang-Yang
-//     512^2 - / - / 7.62 / 7.12, 816^2 - / - / 8.2 / 11.1, 1200^2 16.8 / 18.1
+//     512^2 - / - / 7.62 / 7.12, 816^2 - / - / 8.2 / 11.1, 1200^2 16.8 / 18.1 (taken
+//     before float phases had one series, which took 800^2 from 6.2 to 5.8 and
+//     1200^2 from 12.7 to 11.6)
 struct Fused {
     int n = 0, m = 1;
     int nx = 0, ny = 0;  // regions

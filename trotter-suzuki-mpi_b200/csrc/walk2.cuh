@@ -558,10 +558,11 @@ __device__ __forceinline__ bool w2_rows(Walk2<V, R> &w, int base, uint32_t ph) {
 }
 
 // One task: strip x segment.  The first and last strips come first: their
-// tasks start with extra set-up (clearing the ring bytes outside the tile),
-// and the lowest task indices go to the blocks the SMs schedule first (the
-// warp scheduler favours older blocks; tasks in the youngest blocks of an SM
-// start and finish last).
+// tasks have more to do (masked bodies in the rotating frame and with 4 cells per
+// lane; ring bytes outside the tile to clear, unless the ring is fresh), and the
+// lowest task indices go to the blocks the SMs schedule first (the warp
+// scheduler favours older blocks; tasks in the youngest blocks of an SM start
+// and finish last).
 template <class V, int R>
 __device__ __forceinline__ void w2_task(Walk2<V, R> &w, const StepArgs<typename V::T> &a, int task) {
     using T = typename V::T;
